@@ -35,6 +35,27 @@ constexpr double kZPlanesDensity = 0.2;
 constexpr long long kForkMinKeys = 300000;
 constexpr int kItemStride = 44;    // per work item: 36 block + 6 rhs + pad
 
+// Work-item sizes left to the library (option 0).  The mixed path keeps fixed
+// sizes: the grouping of its FP32 sums is part of its results.  The FP64 path
+// is bound by its FP64 pipe (64 cycles an instruction and warp), so a small
+// problem is cut finer, until its items, image lists and key chunks fill the
+// 608 warp schedulers; its sizes depend on the problem alone, so its bits
+// are the same in any batch.  Below 64 (two entries a lane) an item's own
+// reduction outweighs its sums.
+inline int auto_item(long long count, long long pieces, int unit, int lo, int hi) {
+  const long long per = (count + pieces * unit - 1) / (pieces * unit) * unit;
+  return int(per < lo ? lo : per > hi ? hi : per);
+}
+inline int pair_item_size(int option, bool mixed, long long pairs) {
+  return option > 0 ? option : mixed ? kPairItem : auto_item(pairs, 608, 32, 64, kPairItem);
+}
+inline int image_item_size(int option, bool mixed, long long keys) {
+  return option > 0 ? option : mixed ? kImageItem : auto_item(keys, 3040, 32, 64, kImageItem / 2);
+}
+inline int key_item_size(int option, bool mixed, long long keys) {
+  return option > 0 ? option : mixed ? kKeyChunk : auto_item(keys, 304, 128, 128, kKeyChunk);
+}
+
 // Per-problem LM state (device).  Written only by the control kernels.
 struct LMState {
   double mu, nu;

@@ -988,12 +988,26 @@ __global__ void __launch_bounds__(kPointChunk) k_point_reduce(DevPlan d) {
   }
 }
 
-// ---------------------------------------------------------------------------
 // image reduce: U_i = sum J_i^T J_i, g_i = sum J_i^T r.  Each image's keys
-// are split into work items of <= kImageItem keys (one warp each, Kahan lane
-// sums in T, warp sum in T); k_image_finalize adds an image's items in order
-// in FP64.
+// are split into work items (one warp each); k_image_finalize adds an image's
+// items in FP64.  The FP32 lanes add with Kahan compensation (up to 16 keys a
+// lane).  The FP64 lanes add plain FMA chains of at most eight keys: the pipe
+// takes 64 cycles an instruction, Kahan sums took three times as many, and
+// with four interleaved sums over the items the error against exact sums
+// is no larger (500 to 20,000 keys: 5.1e-17 to 6.3e-17 of the sum of
+// magnitudes, before 5.3e-17 to 1.1e-16, root mean square).
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void add_dot2(float& acc, float& cmp, float x0, float y0, float x1, float y1) {
+  const float term = x0 * y0 + x1 * y1;
+  const float y = term - cmp;
+  const float t = acc + y;
+  cmp = (t - acc) - y;
+  acc = t;
+}
+__device__ __forceinline__ void add_dot2(double& acc, double&, double x0, double y0, double x1, double y1) {
+  acc = fma(x1, y1, fma(x0, y0, acc));
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) k_image_reduce(DevPlan d) {
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1003,7 +1017,7 @@ __global__ void __launch_bounds__(256) k_image_reduce(DevPlan d) {
   const LMState& st = d.state[it.w];
   if (!st.relin || !st.active) return;
   const T* __restrict__ JR = tptr<T>(d.JR[st.parity]);
-  T acc[27], cmp[27];
+  T acc[27], cmp[27];   // (cmp: FP32 only)
 #pragma unroll
   for (int e = 0; e < 27; ++e) { acc[e] = T(0); cmp[e] = T(0); }
   for (int q = it.y + lane; q < it.z; q += 32) {
@@ -1016,29 +1030,20 @@ __global__ void __launch_bounds__(256) k_image_reduce(DevPlan d) {
     for (int a = 0; a < 6; ++a) {
 #pragma unroll
       for (int b = a; b < 6; ++b) {
-        const T term = ji[a] * ji[b] + ji[6 + a] * ji[6 + b];
-        const T y = term - cmp[e];
-        const T t = acc[e] + y;
-        cmp[e] = (t - acc[e]) - y;
-        acc[e] = t;
+        add_dot2(acc[e], cmp[e], ji[a], ji[b], ji[6 + a], ji[6 + b]);
         ++e;
       }
     }
 #pragma unroll
-    for (int a = 0; a < 6; ++a) {
-      const T term = ji[a] * rec[18] + ji[6 + a] * rec[19];
-      const T y = term - cmp[21 + a];
-      const T t = acc[21 + a] + y;
-      cmp[21 + a] = (t - acc[21 + a]) - y;
-      acc[21 + a] = t;
-    }
+    for (int a = 0; a < 6; ++a) add_dot2(acc[21 + a], cmp[21 + a], ji[a], rec[18], ji[6 + a], rec[19]);
   }
-  double* out = d.img_item_partial + 28LL * wid;
+  if constexpr (sizeof(T) == sizeof(float)) {
 #pragma unroll
-  for (int e = 0; e < 27; ++e) {
-    const T v = warp_sum_t(T(acc[e] - cmp[e]));
-    if (lane == e) out[e] = double(v);
+    for (int e = 0; e < 27; ++e) acc[e] -= cmp[e];
   }
+  int base, count;
+  warp_scatter_sums<27>(acc, lane, base, count);
+  if (count > 0) d.img_item_partial[28LL * wid + base] = double(acc[0]);
 }
 
 __global__ void __launch_bounds__(256) k_image_finalize(DevPlan d) {
@@ -1050,8 +1055,19 @@ __global__ void __launch_bounds__(256) k_image_finalize(DevPlan d) {
   if (!st.relin || !st.active) return;
   const int ib = d.img_item_off[img], ie = d.img_item_off[img + 1];
   double v = 0.0;
-  if (lane < 27)
-    for (int t = ib; t < ie; ++t) v += d.img_item_partial[28LL * t + lane];
+  if (lane < 27) {
+    const double* part = d.img_item_partial + lane;
+    if (d.precision == GBA_PRECISION_MIXED) {
+      for (int t = ib; t < ie; ++t) v += part[28LL * t];
+    } else {   // finer items (image_item_size): four interleaved sums
+      double s[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int t = ib; t < ie; t += 4)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (t + u < ie) s[u] += part[28LL * (t + u)];
+      v = (s[0] + s[1]) + (s[2] + s[3]);
+    }
+  }
   // lane e holds entry e of (upper U in row order, then g)
   double* U = d.U + 36LL * img;
   double dmax = 0.0, gmax = 0.0;

@@ -707,10 +707,15 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
     std::vector<double> prior_y, prior_info;
     long long n_pairs = 0;             // key pairs (blocks built on the device)
   };
-  // work-item sizes of the Schur assembly and the image reduction
-  const int pair_item = opt.pair_item > 0 ? opt.pair_item : kPairItem;
-  const int image_item = opt.image_item > 0 ? opt.image_item : kImageItem;
-  const int key_item = opt.key_item > 0 ? opt.key_item : kKeyChunk;
+  std::vector<Piece> pieces(nprob);
+  // work-item sizes of the Schur assembly, the image reduction and the key
+  // chunks, per problem
+  auto pair_item_of = [&](int q) {
+    return pair_item_size(opt.pair_item, mixed, pieces[q].blk_off.empty() ? 0 : pieces[q].blk_off.back());
+  };
+  auto key_item_of = [&](int q) { return key_item_size(opt.key_item, mixed, problems[q].number_of_keys); };
+  int max_key_item = 1;
+  for (int q = 0; q < nprob; ++q) max_key_item = std::max(max_key_item, key_item_of(q));
   // plans without free cameras count, number and place their key pairs on
   // the device (GBA_HOST_PAIRS=1 keeps the host build, for comparison); the
   // per-code tables take 12 bytes per (image, image) entry of every problem
@@ -718,7 +723,6 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
   for (int q = 0; q < nprob; ++q) codes += (long long)prob[q].num_ext * prob[q].num_ext;
   const bool dev_blocks = !any_free && nprob <= 65535 && codes <= (1LL << 26) &&
                           std::getenv("GBA_HOST_PAIRS") == nullptr;
-  std::vector<Piece> pieces(nprob);
   // fine phases of a single problem's build (GBA_BUILD_TIMING)
   auto sub = [&](const char* name) {
     if (timing && nprob == 1) phase(name);
@@ -864,6 +868,7 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
       });
       for (int i = 1; i <= ni; ++i) img_key_off[ib + i] = int(kb + ic[i]);   // entry ib: the caller
       out.img_item_cnt.assign(ni, 0);
+      const int image_item = image_item_size(opt.image_item, mixed, nk);
       for (int i = 0; i < ni; ++i) {
         const int q0 = int(kb + ic[i]), q1 = int(kb + ic[i + 1]);
         for (int qq = q0; qq < q1; qq += image_item) {
@@ -1203,6 +1208,7 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
     b.recs += (long long)pc.rec_ext.size();
     const long long nblk = (long long)pc.blk_ij.size();
     b.blocks += nblk;
+    const int pair_item = pair_item_of(q), key_item = key_item_of(q);
     for (long long t = 0; t < nblk; ++t) {
       const long long cntp = pc.blk_off[t + 1] - pc.blk_off[t];
       b.items += std::max<long long>(1, (cntp + pair_item - 1) / pair_item);
@@ -1299,6 +1305,7 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
     pi.block_begin = block_begin;
     pi.num_blocks = nblk;
     pi.item_begin = int(b.items);
+    const int pair_item = pair_item_of(q), key_item = key_item_of(q);
     long long it = b.items;
     for (int t = 0; t < nblk; ++t) {
       const long long s0 = b.pairs + pc.blk_off[t], s1 = b.pairs + pc.blk_off[t + 1];
@@ -1668,7 +1675,7 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
   D.blk_map_off = arena.upload(blk_map_off);
   D.item_partial = arena.alloc<double>(size_t(kItemStride) * std::max<size_t>(items.size(), 1));
   D.n_key_chunks = int(key_chunks.size());
-  D.key_z_split = (key_item + 255) / 256;   // one key per thread of the Z kernel
+  D.key_z_split = (max_key_item + 255) / 256;   // one key per thread of the Z kernel
   D.n_pt_chunks = int(pt_chunks.size());
   D.n_img_chunks = int(img_chunks.size());
   D.key_chunks = arena.upload(key_chunks);
