@@ -343,21 +343,100 @@ __device__ void rodrigues_coeffs(double theta, double& ct, double& s, double& c,
 // from the intrinsic mask hold the identity values (0 / f=1 s=0 c=0 a=1),
 // which reproduce the reference's per-mask projection exactly.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void project64(const double* R, const double* X, const double* cam,
-                                          double& u, double& v) {
-  double y0 = R[0] * X[0] + R[1] * X[1] + R[2] * X[2] + R[9];
-  double y1 = R[3] * X[0] + R[4] * X[1] + R[5] * X[2] + R[10];
-  double y2 = R[6] * X[0] + R[7] * X[1] + R[8] * X[2] + R[11];
-  const double iz = 1.0 / y2;
-  double n0 = y0 * iz, n1 = y1 * iz;
-  double r2 = n0 * n0 + n1 * n1;
-  double coeff = cam[0] * r2 + cam[1] * (r2 * r2) + cam[2] * (r2 * r2 * r2);
-  double dx = coeff * n0 + (2.0 * cam[3] * n0 * n1 + cam[4] * (r2 + 2.0 * n0 * n0));
-  double dy = coeff * n1 + (2.0 * cam[4] * n0 * n1 + cam[3] * (r2 + 2.0 * n1 * n1));
-  n0 += dx;
-  n1 += dy;
-  u = cam[5] * n0 + cam[6] * n1 + cam[7];
-  v = cam[5] * cam[9] * n1 + cam[8];
+// The FP64 pipe takes 64 cycles an instruction and warp (76 with all four
+// schedulers busy), so everything here is written as FMAs, the camera's
+// absent terms are left out (their parameters are tested as integers), and
+// the Jacobian reuses the projection's terms.
+struct Proj64 {
+  double w[3];          // R X
+  double iz, n0, n1;    // 1 / depth, the undistorted normalized key
+  double r2, q;         // n0^2 + n1^2, 1 + radial coefficient
+  double e0, e1;        // the distorted normalized key
+  double u, v;          // the image key
+};
+
+__device__ __forceinline__ bool nonzero64(double x) { return (__double_as_longlong(x) << 1) != 0; }
+
+__device__ __forceinline__ void project64(const double* R, const double* X, const double* cam, Proj64& p) {
+#pragma unroll
+  for (int m = 0; m < 3; ++m) p.w[m] = fma(R[3 * m + 2], X[2], fma(R[3 * m + 1], X[1], R[3 * m] * X[0]));
+  p.iz = 1.0 / (p.w[2] + R[11]);
+  p.n0 = (p.w[0] + R[9]) * p.iz;
+  p.n1 = (p.w[1] + R[10]) * p.iz;
+  p.r2 = fma(p.n1, p.n1, p.n0 * p.n0);
+  p.q = 1.0;
+  double e0 = p.n0, e1 = p.n1;
+  if (nonzero64(cam[0]) || nonzero64(cam[1]) || nonzero64(cam[2])) {
+    const double c = p.r2 * fma(p.r2, fma(p.r2, cam[2], cam[1]), cam[0]);
+    p.q = __dadd_rn(1.0, c);   // (never contracted: the same bits in every caller)
+    e0 = fma(c, e0, e0);
+    e1 = fma(c, e1, e1);
+  }
+  if (nonzero64(cam[3]) || nonzero64(cam[4])) {
+    const double x2 = p.n0 + p.n0, xy2 = x2 * p.n1;
+    e0 = fma(cam[3], xy2, fma(cam[4], fma(x2, p.n0, p.r2), e0));
+    e1 = fma(cam[4], xy2, fma(cam[3], fma(p.n1 + p.n1, p.n1, p.r2), e1));
+  }
+  p.e0 = e0;
+  p.e1 = e1;
+  p.u = fma(cam[5], e0, cam[7]);
+  if (nonzero64(cam[6])) p.u = fma(cam[6], e1, p.u);
+  p.v = fma(cam[5] * cam[9], e1, cam[8]);
+}
+
+// The 2x3 point block jp and the 2x6 image block ji of a key from its
+// projection.  With M = d(u, v) / d(n0, n1) (distortion and intrinsics) and
+// b = M [iz 0 -n0 iz; 0 iz -n1 iz] = d(u, v) / d(camera point): the
+// translation columns are b, jp = b R, and as d(R X) / dr = -[R X]x Jl with
+// the left Jacobian Jl of the image's angle-axis vector, the rotation columns
+// are (R X x b) Jl for each row of b.  These are the derivatives of the
+// reference's chain (:334-524) in 70 FP64 instructions instead of about 420.
+// l00, l10, l11 and sw whiten and weight M (and so every column); unit false
+// when they are the identity.
+__device__ __forceinline__ void jacobian64(const double* R, const double* Jl, const double* cam, const Proj64& p,
+                                           bool unit, double l00, double l10, double l11, double sw, double* jp,
+                                           double* ji) {
+  double e00 = p.q, e01 = 0.0, e11 = p.q;
+  if (nonzero64(cam[0]) || nonzero64(cam[1]) || nonzero64(cam[2])) {
+    const double dc = 2.0 * fma(p.r2, fma(p.r2, 3.0 * cam[2], 2.0 * cam[1]), cam[0]);
+    const double t = dc * p.n0;
+    e00 = fma(t, p.n0, e00);
+    e01 = t * p.n1;
+    e11 = fma(dc * p.n1, p.n1, e11);
+  }
+  if (nonzero64(cam[3]) || nonzero64(cam[4])) {
+    const double x1 = 2.0 * cam[3], x2 = 2.0 * cam[4];
+    e00 = fma(x1, p.n1, fma(3.0 * x2, p.n0, e00));
+    e01 = fma(x1, p.n0, fma(x2, p.n1, e01));
+    e11 = fma(x2, p.n0, fma(3.0 * x1, p.n1, e11));
+  }
+  const double f = cam[5], fa = cam[5] * cam[9];
+  double m00 = f * e00, m01 = f * e01, m10 = fa * e01, m11 = fa * e11;
+  if (nonzero64(cam[6])) {
+    m00 = fma(cam[6], e01, m00);
+    m01 = fma(cam[6], e11, m01);
+  }
+  if (!unit) {
+    m00 = sw * fma(l00, m00, l10 * m10);
+    m01 = sw * fma(l00, m01, l10 * m11);
+    m10 = sw * (l11 * m10);
+    m11 = sw * (l11 * m11);
+  }
+  const double b[2][3] = {{m00 * p.iz, m01 * p.iz, 0.0}, {m10 * p.iz, m11 * p.iz, 0.0}};
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const double b0 = b[r][0], b1 = b[r][1], b2 = -fma(b0, p.n0, b1 * p.n1);
+    const double c0 = fma(p.w[1], b2, -(p.w[2] * b1)), c1 = fma(p.w[2], b0, -(p.w[0] * b2)),
+                 c2 = fma(p.w[0], b1, -(p.w[1] * b0));
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      jp[3 * r + j] = fma(b2, R[6 + j], fma(b1, R[3 + j], b0 * R[j]));
+      ji[6 * r + j] = fma(c2, Jl[6 + j], fma(c1, Jl[3 + j], c0 * Jl[j]));
+    }
+    ji[6 * r + 3] = b0;
+    ji[6 * r + 4] = b1;
+    ji[6 * r + 5] = b2;
+  }
 }
 
 // Analytical Jacobian of one key in precision T: jp 2x3, ji 2x6 (row-major).
@@ -482,6 +561,25 @@ __device__ __forceinline__ void camera_jacobian(T n0, T n1, const T* cam, T* jc)
   jc[9] = T(0);  jc[19] = f * e1;   // a
 }
 
+// The same in FP64 from the key's projection (every rounding explicit, so the
+// bits do not depend on the calling kernel).
+__device__ __forceinline__ void camera_jacobian64(const Proj64& p, const double* cam, double* jc) {
+  const double r4 = p.r2 * p.r2, r6 = r4 * p.r2, x2 = p.n0 + p.n0, xy2 = x2 * p.n1;
+  const double f = cam[5], sk = cam[6], a = cam[9], fa = f * a;
+  const double de0[5] = {p.r2 * p.n0, r4 * p.n0, r6 * p.n0, xy2, fma(x2, p.n0, p.r2)};
+  const double de1[5] = {p.r2 * p.n1, r4 * p.n1, r6 * p.n1, fma(p.n1 + p.n1, p.n1, p.r2), xy2};
+#pragma unroll
+  for (int m = 0; m < 5; ++m) {
+    jc[m] = fma(sk, de1[m], f * de0[m]);
+    jc[10 + m] = fa * de1[m];
+  }
+  jc[5] = p.e0;  jc[15] = a * p.e1;   // f
+  jc[6] = p.e1;  jc[16] = 0.0;        // s
+  jc[7] = 1.0;   jc[17] = 0.0;        // cx
+  jc[8] = 0.0;   jc[18] = 1.0;        // cy
+  jc[9] = 0.0;   jc[19] = f * p.e1;   // a
+}
+
 // Column of the full ten [k1 k2 k3 d1 d2 f s cx cy a] holding a camera's
 // computed parameter m, or -1 past its count.
 __host__ __device__ __forceinline__ int cam_full_col(unsigned mask, int m) {
@@ -602,9 +700,20 @@ __device__ void image_prep_one(const DevPlan& d, int i, int par) {
     for (int j = 0; j < 12; ++j) Rf[j] = ff_split(R[j]);
   }
   T* IL = tptr_mut<T>(d.img_lin[par]) + 12LL * i;
-  IL[0] = T(r0); IL[1] = T(r1); IL[2] = T(r2);
-  IL[3] = T(x[3]); IL[4] = T(x[4]); IL[5] = T(x[5]);
-  IL[6] = T(ct); IL[7] = T(s); IL[8] = T(c); IL[9] = T(a1); IL[10] = T(a2); IL[11] = T(0);
+  if constexpr (sizeof(T) == sizeof(double)) {
+    // left Jacobian of the angle-axis vector: s I + c [r]x + b r r^T, b =
+    // (1 - s) / theta^2 (jacobian64; its rows, then padding)
+    const double t2 = theta * theta;
+    const double b = theta < 1e-2 ? 1.0 / 6.0 - t2 / 120.0 + t2 * t2 / 5040.0 : (1.0 - s) / t2;
+    IL[0] = s + b * r0 * r0;       IL[1] = b * r0 * r1 - c * r2;  IL[2] = b * r0 * r2 + c * r1;
+    IL[3] = b * r1 * r0 + c * r2;  IL[4] = s + b * r1 * r1;       IL[5] = b * r1 * r2 - c * r0;
+    IL[6] = b * r2 * r0 - c * r1;  IL[7] = b * r2 * r1 + c * r0;  IL[8] = s + b * r2 * r2;
+    IL[9] = IL[10] = IL[11] = 0.0;
+  } else {
+    IL[0] = T(r0); IL[1] = T(r1); IL[2] = T(r2);
+    IL[3] = T(x[3]); IL[4] = T(x[4]); IL[5] = T(x[5]);
+    IL[6] = T(ct); IL[7] = T(s); IL[8] = T(c); IL[9] = T(a1); IL[10] = T(a2); IL[11] = T(0);
+  }
 }
 
 // which = 0: the current x of active problems (at init); 1: the candidate of
@@ -663,48 +772,57 @@ __global__ void __launch_bounds__(256) k_cons_cost(DevPlan d, int which) {
 // camera at that parity; rw0, rw1, sw the key's weighted residual and the
 // square root of its IRLS weight.
 // ---------------------------------------------------------------------------
+// The camera block jc of key k (free cameras), whitened and weighted as the
+// others, into JC.
+__device__ __forceinline__ float whiten_u(float l00, float a, float l10, float b) { return l00 * a + l10 * b; }
+__device__ __forceinline__ double whiten_u(double l00, double a, double l10, double b) { return fma(l00, a, l10 * b); }
+
 template <typename T>
-__device__ __forceinline__ void linearize_key(const DevPlan& d, int k, int par, int fix, const T* X, const T* il,
-                                              const T* cam, T rw0, T rw1, T sw) {
-  T jp[6], ji[12], nrm[2];
-  key_jacobian<T>(X, il, cam, jp, ji, nrm);
+__device__ __forceinline__ void linearize_cam(const DevPlan& d, int k, int par, T* jc, T sw) {
+  T l00 = T(1), l10 = T(0), l11 = T(1);
+  if (d.key_wl) {
+    l00 = T(__ldg(d.key_wl + 3LL * k));
+    l10 = T(__ldg(d.key_wl + 3LL * k + 1));
+    l11 = T(__ldg(d.key_wl + 3LL * k + 2));
+  }
+#pragma unroll
+  for (int m = 0; m < 10; ++m) {
+    const T a = jc[m], b = jc[10 + m];
+    jc[m] = whiten_u(l00, a, l10, b) * sw;
+    jc[10 + m] = l11 * b * sw;
+  }
+  store_vec<20>(tptr_mut<T>(d.JC[par]) + 20LL * k, jc);
+}
+
+__device__ __forceinline__ void linearize_key(const DevPlan& d, int k, int par, int fix, const float* X,
+                                              const float* il, const float* cam, float rw0, float rw1, float sw) {
+  float jp[6], ji[12], nrm[2];
+  key_jacobian<float>(X, il, cam, jp, ji, nrm);
   if (fix & 1) {   // fixed points: no point columns
 #pragma unroll
-    for (int m = 0; m < 6; ++m) jp[m] = T(0);
+    for (int m = 0; m < 6; ++m) jp[m] = 0.0f;
   }
   if (fix & 2) {   // fixed images: no image columns
 #pragma unroll
-    for (int m = 0; m < 12; ++m) ji[m] = T(0);
+    for (int m = 0; m < 12; ++m) ji[m] = 0.0f;
   }
-  if (d.free_cams) {   // the camera block, whitened and weighted as the others
-    T jc[20];
-    camera_jacobian<T>(nrm[0], nrm[1], cam, jc);
-    T l00 = T(1), l10 = T(0), l11 = T(1);
-    if (d.key_wl) {
-      l00 = T(__ldg(d.key_wl + 3LL * k));
-      l10 = T(__ldg(d.key_wl + 3LL * k + 1));
-      l11 = T(__ldg(d.key_wl + 3LL * k + 2));
-    }
-#pragma unroll
-    for (int m = 0; m < 10; ++m) {
-      const T a = jc[m], b = jc[10 + m];
-      jc[m] = (l00 * a + l10 * b) * sw;
-      jc[10 + m] = l11 * b * sw;
-    }
-    store_vec<20>(tptr_mut<T>(d.JC[par]) + 20LL * k, jc);
+  if (d.free_cams) {
+    float jc[20];
+    camera_jacobian<float>(nrm[0], nrm[1], cam, jc);
+    linearize_cam<float>(d, k, par, jc, sw);
   }
   if (d.key_wl) {
-    const T l00 = T(__ldg(d.key_wl + 3LL * k)), l10 = T(__ldg(d.key_wl + 3LL * k + 1)),
-            l11 = T(__ldg(d.key_wl + 3LL * k + 2));
+    const float l00 = float(__ldg(d.key_wl + 3LL * k)), l10 = float(__ldg(d.key_wl + 3LL * k + 1)),
+                l11 = float(__ldg(d.key_wl + 3LL * k + 2));
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-      const T a = jp[m], b = jp[3 + m];
+      const float a = jp[m], b = jp[3 + m];
       jp[m] = (l00 * a + l10 * b) * sw;
       jp[3 + m] = l11 * b * sw;
     }
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
-      const T a = ji[m], b = ji[6 + m];
+      const float a = ji[m], b = ji[6 + m];
       ji[m] = (l00 * a + l10 * b) * sw;
       ji[6 + m] = l11 * b * sw;
     }
@@ -714,39 +832,78 @@ __device__ __forceinline__ void linearize_key(const DevPlan& d, int k, int par, 
 #pragma unroll
     for (int m = 0; m < 12; ++m) ji[m] *= sw;
   }
-  T rec[kJRStride];
+  float rec[kJRStride];
 #pragma unroll
   for (int m = 0; m < 6; ++m) rec[m] = jp[m];
 #pragma unroll
   for (int m = 0; m < 12; ++m) rec[6 + m] = ji[m];
   rec[18] = rw0;
   rec[19] = rw1;
-  store_vec<kJRStride>(tptr_mut<T>(d.JR[par]) + (long long)kJRStride * k, rec);
+  store_vec<kJRStride>(tptr_mut<float>(d.JR[par]) + (long long)kJRStride * k, rec);
+}
+
+// The FP64 record of key k from its projection p and the rotation R of its image.
+__device__ __forceinline__ void linearize_key64(const DevPlan& d, int k, int img, int par, int fix, const double* R,
+                                                const double* cam, const Proj64& p, double rw0, double rw1,
+                                                double sw) {
+  double Jl[10], rec[kJRStride];
+  load_vec<10>(tptr<double>(d.img_lin[par]) + 12LL * img, Jl);
+  double l00 = 1.0, l10 = 0.0, l11 = 1.0;
+  if (d.key_wl) {
+    l00 = __ldg(d.key_wl + 3LL * k);
+    l10 = __ldg(d.key_wl + 3LL * k + 1);
+    l11 = __ldg(d.key_wl + 3LL * k + 2);
+  }
+  const bool unit = !d.key_wl && __double_as_longlong(sw) == __double_as_longlong(1.0);
+  jacobian64(R, Jl, cam, p, unit, l00, l10, l11, sw, rec, rec + 6);
+  if (fix & 1) {   // fixed points: no point columns
+#pragma unroll
+    for (int m = 0; m < 6; ++m) rec[m] = 0.0;
+  }
+  if (fix & 2) {   // fixed images: no image columns
+#pragma unroll
+    for (int m = 6; m < 18; ++m) rec[m] = 0.0;
+  }
+  if (d.free_cams) {
+    double jc[20];
+    camera_jacobian64(p, cam, jc);
+    linearize_cam<double>(d, k, par, jc, sw);
+  }
+  rec[18] = rw0;
+  rec[19] = rw1;
+  store_vec<kJRStride>(tptr_mut<double>(d.JR[par]) + (long long)kJRStride * k, rec);
 }
 
 // The records of a key chunk at parity par, one key per thread.
 template <typename T>
 __device__ __forceinline__ void linearize_chunk(const DevPlan& d, const Chunk& ch, int par) {
   const double* __restrict__ xp = d.x_pt[par];
-  const T* __restrict__ IL = tptr<T>(d.img_lin[par]);
   const T* __restrict__ rwb = tptr<T>(d.RW[par]);
   const int fix = d.prob[ch.prob].fix;
   for (int k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) {
     const int img = __ldg(d.key_img + k), pt = __ldg(d.key_pt + k);
-    T X[3];
-    if (sizeof(T) == sizeof(float) && d.x_ff[par]) {   // mixed: high part of the mirror
-      const float2* xf = d.x_ff[par] + 3LL * pt;
-      X[0] = T(xf[0].x); X[1] = T(xf[1].x); X[2] = T(xf[2].x);
-    } else {
-      X[0] = T(xp[3LL * pt]); X[1] = T(xp[3LL * pt + 1]); X[2] = T(xp[3LL * pt + 2]);
-    }
-    T il[12];
-    load_vec<12>(IL + 12LL * img, il);
     T cam[10];
     load_cam<T>(d, par, __ldg(d.img_cam + img), cam);
     T rw[4];
     load_vec<4>(rwb + 4LL * k, rw);
-    linearize_key<T>(d, k, par, fix, X, il, cam, rw[0], rw[1], rw[2]);
+    if constexpr (sizeof(T) == sizeof(double)) {
+      double R[12];
+      load_vec<12>(d.img_rot[par] + 12LL * img, R);
+      const double X[3] = {xp[3LL * pt], xp[3LL * pt + 1], xp[3LL * pt + 2]};
+      Proj64 p;
+      project64(R, X, cam, p);
+      linearize_key64(d, k, img, par, fix, R, cam, p, rw[0], rw[1], rw[2]);
+    } else {
+      float X[3], il[12];
+      if (d.x_ff[par]) {   // mixed: high part of the mirror
+        const float2* xf = d.x_ff[par] + 3LL * pt;
+        X[0] = xf[0].x; X[1] = xf[1].x; X[2] = xf[2].x;
+      } else {
+        X[0] = float(xp[3LL * pt]); X[1] = float(xp[3LL * pt + 1]); X[2] = float(xp[3LL * pt + 2]);
+      }
+      load_vec<12>(tptr<float>(d.img_lin[par]) + 12LL * img, il);
+      linearize_key(d, k, par, fix, X, il, cam, rw[0], rw[1], rw[2]);
+    }
   }
 }
 
@@ -760,51 +917,58 @@ __global__ void __launch_bounds__(256) k_linearize_keys(DevPlan d) {
   linearize_chunk<T>(d, ch, st.parity);
 }
 
-template <typename T>
+// FP64 cost, and for a candidate its Jacobian records from the same
+// projection (each key's residual goes into its record; RW is written only
+// for a separate linearization).  Bound by the FP64 pipe: about 115
+// instructions a key (480 with the chain kept apart for each column: 24
+// windows of 0.95 M keys in all 27.6 -> 22.7 ms a solve, grid 4.57 -> 4.0 ms
+// an iteration).
 __global__ void __launch_bounds__(256) k_cost(DevPlan d, int which) {
   __shared__ double red[32];
   const Chunk ch = d.key_chunks[blockIdx.x];
   const LMState& st = d.state[ch.prob];
   if (which == 0 ? !st.active : !st.evaluate) return;
   const int par = which ? 1 - st.parity : st.parity;
+  const bool records = which == 1 && d.fuse_lin;
+  const int fix = d.prob[ch.prob].fix;
   const double* __restrict__ xp = d.x_pt[par];
-  const double* __restrict__ rot = d.img_rot[par];
-  T* __restrict__ rw = tptr_mut<T>(d.RW[par]);
+  double* __restrict__ rw = tptr_mut<double>(d.RW[par]);
   double acc = 0.0, acc_raw = 0.0;
   for (int k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) {
     const int img = __ldg(d.key_img + k), pt = __ldg(d.key_pt + k);
-    double R[12];
-#pragma unroll
-    for (int j = 0; j < 12; ++j) R[j] = rot[12LL * img + j];
-    double X[3] = {xp[3LL * pt], xp[3LL * pt + 1], xp[3LL * pt + 2]};
-    double cam[10];
-    const int ci = __ldg(d.img_cam + img);
-#pragma unroll
-    for (int j = 0; j < 10; ++j) cam[j] = d.cam64[par][10 * ci + j];
-    double u, v;
-    project64(R, X, cam, u, v);
+    double R[12], cam[10];
+    // (written by an earlier launch: read-only here)
+    load_vec<12>(d.img_rot[par] + 12LL * img, R);
+    const double X[3] = {xp[3LL * pt], xp[3LL * pt + 1], xp[3LL * pt + 2]};
+    load_vec<10>(d.cam64[par] + 10LL * __ldg(d.img_cam + img), cam);
+    Proj64 p;
+    project64(R, X, cam, p);
     const double2 ob = __ldg(d.key_obs + k);
-    double e0 = u - ob.x, e1 = v - ob.y;   // r = f(x) - y
-    acc_raw += e0 * e0 + e1 * e1;
+    double e0 = p.u - ob.x, e1 = p.v - ob.y;   // r = f(x) - y
+    double sq = fma(e1, e1, e0 * e0);
+    acc_raw += sq;
     if (d.key_wl) {
       const double l00 = __ldg(d.key_wl + 3LL * k), l10 = __ldg(d.key_wl + 3LL * k + 1),
                    l11 = __ldg(d.key_wl + 3LL * k + 2);
-      double w0 = l00 * e0 + l10 * e1;
+      e0 = fma(l00, e0, l10 * e1);
       e1 = l11 * e1;
-      e0 = w0;
+      sq = fma(e1, e1, e0 * e0);
     }
-    const double sq = e0 * e0 + e1 * e1;
-    double rho, w;
-    loss_eval(d.loss, d.huber_delta, sq, rho, w);
+    double rho = sq, w, sw = 1.0;
+    if (d.loss != GBA_LOSS_TRIVIAL) {
+      loss_eval(d.loss, d.huber_delta, sq, rho, w);
+      if (w != 1.0) {
+        sw = sqrt(w);
+        e0 *= sw;
+        e1 *= sw;
+      }
+    }
     acc += rho;
-    const double sw = (w == 1.0) ? 1.0 : sqrt(w);
-    T out[4] = {T(e0 * sw), T(e1 * sw), T(sw), T(0)};
-    store_vec<4>(rw + 4LL * k, out);
-    if (which == 1 && d.fuse_lin) {   // the candidate's Jacobian records, used if it is accepted
-      T Xl[3] = {T(X[0]), T(X[1]), T(X[2])}, il[12], cl[10];
-      load_vec<12>(tptr<T>(d.img_lin[par]) + 12LL * img, il);
-      load_cam<T>(d, par, ci, cl);
-      linearize_key<T>(d, k, par, d.prob[ch.prob].fix, Xl, il, cl, out[0], out[1], out[2]);
+    if (records) {   // the candidate's Jacobian records, used if it is accepted
+      linearize_key64(d, k, img, par, fix, R, cam, p, e0, e1, sw);
+    } else {
+      const double out[4] = {e0, e1, sw, 0.0};
+      store_vec<4>(rw + 4LL * k, out);
     }
   }
   const double tot = block_sum(acc, red);
@@ -3518,10 +3682,10 @@ __global__ void k_vector_function(DevPlan d, double* y) {
   double X[3] = {xp[0], xp[1], xp[2]};
   double cam[10];
   for (int j = 0; j < 10; ++j) cam[j] = d.cam64[par][10 * d.img_cam[img] + j];
-  double u, v;
-  project64(R, X, cam, u, v);
-  y[2LL * k] = u;
-  y[2LL * k + 1] = v;
+  Proj64 p;
+  project64(R, X, cam, p);
+  y[2LL * k] = p.u;
+  y[2LL * k + 1] = p.v;
 }
 
 template <typename T>
@@ -3531,18 +3695,28 @@ __global__ void k_jacobian_out(DevPlan d, double* jp_out, double* ji_out, double
   const int img = d.key_img[k], pt = d.key_pt[k];
   const int par = d.state[d.img_prob[img]].parity;
   const double* xp = d.x_pt[par] + 3LL * pt;
-  const T X[3] = {T(xp[0]), T(xp[1]), T(xp[2])};
-  T il[12];
-  for (int j = 0; j < 12; ++j) il[j] = tptr<T>(d.img_lin[par])[12LL * img + j];
   T cam[10];
   load_cam<T>(d, par, d.img_cam[img], cam);
-  T jp[6], ji[12], nrm[2];
-  key_jacobian<T>(X, il, cam, jp, ji, nrm);
+  T jp[6], ji[12], jc[20];
+  if constexpr (sizeof(T) == sizeof(double)) {
+    double R[12], Jl[9];
+    for (int j = 0; j < 12; ++j) R[j] = d.img_rot[par][12LL * img + j];
+    for (int j = 0; j < 9; ++j) Jl[j] = tptr<double>(d.img_lin[par])[12LL * img + j];
+    Proj64 p;
+    project64(R, xp, cam, p);
+    jacobian64(R, Jl, cam, p, true, 1.0, 0.0, 1.0, 1.0, jp, ji);
+    camera_jacobian64(p, cam, jc);
+  } else {
+    T nrm[2];
+    const T X[3] = {T(xp[0]), T(xp[1]), T(xp[2])};
+    T il[12];
+    for (int j = 0; j < 12; ++j) il[j] = tptr<T>(d.img_lin[par])[12LL * img + j];
+    key_jacobian<T>(X, il, cam, jp, ji, nrm);
+    camera_jacobian<T>(nrm[0], nrm[1], cam, jc);
+  }
   for (int j = 0; j < 6; ++j) jp_out[6LL * k + j] = double(jp[j]);
   for (int j = 0; j < 12; ++j) ji_out[12LL * k + j] = double(ji[j]);
   if (jc_out) {   // all ten columns; the host keeps the computed ones
-    T jc[20];
-    camera_jacobian<T>(nrm[0], nrm[1], cam, jc);
     for (int j = 0; j < 20; ++j) jc_out[20LL * k + j] = double(jc[j]);
   }
 }
@@ -3646,7 +3820,7 @@ int launch_cost(const DevPlan& d, int which, cudaStream_t s) {
     if (d.precision == GBA_PRECISION_MIXED)
       k_cost_ff<<<d.n_key_chunks, 256, 0, s>>>(d, which);
     else
-      k_cost<double><<<d.n_key_chunks, 256, 0, s>>>(d, which);
+      k_cost<<<d.n_key_chunks, 256, 0, s>>>(d, which);
     ++n;
   }
   return n;
