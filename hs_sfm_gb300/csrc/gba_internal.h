@@ -172,6 +172,8 @@ struct DevPlan {
   int* factor_flag;          // [B] 0 ok, 1 not positive definite, 2 a bounded wait ran out
   // dataflow factorization (one problem; df_grid == 0: per-column launches)
   int df_grid, df_max_own;
+  int df_rows;               // CTAs 0 .. df_rows - 1 own the last tiles of their row alone (nt, or 0)
+  int df_helpers;            // the next df_helpers own the tiles left of those (nt, or 0)
   const int* df_own_off;     // [df_grid + 1] owned tiles of each CTA
   const int2* df_own;        // (i, j) per owned tile, sorted by (j, i) within a CTA
   unsigned* df_flags;        // [nt * nt] epoch at which tile (i, j) was published
@@ -326,7 +328,7 @@ int prepare_cholesky_solve(int max_nt, int precision);
 bool prepare_chol_small(int max_nt, int precision);
 // Tile ownership of the dataflow factorization of an nt-tile system for this
 // device, or false when it does not fit in shared memory.
-bool dataflow_layout(int nt, bool mixed, int device, int* grid, int* max_own,
+bool dataflow_layout(int nt, bool mixed, int device, int* grid, int* max_own, int* rows, int* helpers,
                      std::vector<int>* own_off, std::vector<int2>* own);
 int launch_backsub(const DevPlan& d, cudaStream_t s);
 int launch_ctrl_step(const DevPlan& d, cudaStream_t s);

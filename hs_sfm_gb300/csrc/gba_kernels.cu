@@ -1959,103 +1959,354 @@ __device__ __forceinline__ void tile_sub_xyt_t(Tile<T>& A, const Tile<T>& X, con
 // A -= X Y^T (32x32x32) by threads 0..127, 8 outputs each.
 template <typename T>
 __device__ __forceinline__ void tile_sub_xyt(Tile<T>& A, const Tile<T>& X, const Tile<T>& Y) {
-  if (threadIdx.x >= 128) return;
-  T s[8];
-  tile_xyt<T>(X, Y, s);
-  const int r = threadIdx.x >> 3, c0 = threadIdx.x & 7;
+  if (threadIdx.x < 128) tile_sub_xyt_t<T>(A, X, Y, threadIdx.x);
+}
+
+__device__ __forceinline__ void load16(const float* p, float* o) {
+  Vec16<float>::unpack(*reinterpret_cast<const float4*>(p), o);
+}
+__device__ __forceinline__ void load16(const double* p, double* o) {
+  Vec16<double>::unpack(*reinterpret_cast<const double2*>(p), o);
+}
+
+// The lower triangle of A -= X X^T (the sums of tile_sub_xyt) by threads
+// 0..127; what lies above the diagonal is not used afterwards.  FP32: the rows
+// above 16 leave their upper half out.  FP64 (bound by its pipe: 64 cycles an
+// instruction and warp): column c's 32 - c rows and column 32 - c's c rows
+// share one warp, so 17 warp columns instead of 32.
+__device__ __forceinline__ void tile_sub_sym(Tile<float>& A, const Tile<float>& X) {
+  const int t = threadIdx.x;
+  if (t >= 128) return;
+  const int r = t >> 3, c0 = t & 7;
+  float s0[2] = {0.0f, 0.0f}, s1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+  for (int q = 0; q < kTile; q += 4) {
+    float x0[4], x1[4];
+    load16(&X[r][q], x0);
+    load16(&X[r + 16][q], x1);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      float y[4];
+      load16(&X[c0 + 8 * u][q], y);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (u < 2) s0[u < 2 ? u : 0] = fmaf(x0[e], y[e], s0[u < 2 ? u : 0]);
+        s1[u] = fmaf(x1[e], y[e], s1[u]);
+      }
+    }
+  }
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    A[r][c0 + 8 * u] -= s[u];
-    A[r + 16][c0 + 8 * u] -= s[4 + u];
+    if (u < 2) A[r][c0 + 8 * u] -= s0[u < 2 ? u : 0];
+    A[r + 16][c0 + 8 * u] -= s1[u];
   }
+}
+// The same by 256 threads: the lower 128 take columns c0 and c0 + 8, the others
+// c0 + 16 and c0 + 24 (of the rows from 16 on).
+__device__ __forceinline__ void tile_sub_sym_half(Tile<float>& A, const Tile<float>& X) {
+  const int t = threadIdx.x & 127, h = threadIdx.x >> 7;
+  const int r = t >> 3, c0 = (t & 7) + 16 * h;
+  float s0[2] = {0.0f, 0.0f}, s1[2] = {0.0f, 0.0f};
+#pragma unroll
+  for (int q = 0; q < kTile; q += 4) {
+    float x0[4], x1[4];
+    if (h == 0) load16(&X[r][q], x0);
+    load16(&X[r + 16][q], x1);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      float y[4];
+      load16(&X[c0 + 8 * u][q], y);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (h == 0) s0[u] = fmaf(x0[e], y[e], s0[u]);
+        s1[u] = fmaf(x1[e], y[e], s1[u]);
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    if (h == 0) A[r][c0 + 8 * u] -= s0[u];
+    A[r + 16][c0 + 8 * u] -= s1[u];
+  }
+}
+__device__ __forceinline__ void tile_sub_sym_half(Tile<double>&, const Tile<double>&) {}   // (FP64 rows keep two tiles)
+__device__ __forceinline__ void tile_sub_sym(Tile<double>& A, const Tile<double>& X) {
+  if (threadIdx.x >= 128) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int c = warp; c <= 16; c += 4) {
+    const bool own = lane >= c;
+    const int row = own ? lane : 32 - c + lane, col = own ? c : 32 - c;
+    if (c == 16 && !own) continue;   // (column 16 is its own partner)
+    double s = 0.0;
+#pragma unroll 4
+    for (int q = 0; q < kTile; q += 2) {
+      double x[2], y[2];
+      load16(&X[row][q], x);
+      load16(&X[col][q], y);
+      s = fma(x[0], y[0], s);
+      s = fma(x[1], y[1], s);
+    }
+    A[row][col] -= s;
+  }
+}
+
+// P = A Li^T for a lower triangular Li (a panel: Li = L_jj^-1) by kWarps warps
+// (this one is the w-th): lane = row, warp w the columns 2 kWarps m + w and
+// 2 kWarps m + 2 kWarps - 1 - w (an even split of the triangle).  The terms
+// past a column's diagonal are zeros and are left out: the sums of tile_xyt
+// in half its products.  P may not be A.
+template <typename T, int kWarps>
+__device__ __forceinline__ void tile_panel(const Tile<T>& A, const Tile<T>& Li, Tile<T>& P, int w, int lane) {
+  constexpr int N = Vec16<T>::N, C = kTile / kWarps;
+  int col[C];
+  T s[C];
+#pragma unroll
+  for (int u = 0; u < C; ++u) {
+    col[u] = kWarps * u + ((u & 1) ? kWarps - 1 - w : w);
+    s[u] = T(0);
+  }
+#pragma unroll
+  for (int q = 0; q < kTile; q += N) {
+    T x[N];
+    load16(&A[lane][q], x);
+#pragma unroll
+    for (int u = 0; u < C; ++u) {
+      if (q > kWarps * (u + 1) - 1) continue;   // (the column's range: col[u] < kWarps (u + 1))
+      if (q <= col[u]) {
+        T y[N];
+        load16(&Li[col[u]][q], y);
+#pragma unroll
+        for (int e = 0; e < N; ++e) s[u] = fma(x[e], y[e], s[u]);
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < C; ++u) P[lane][col[u]] = s[u];
 }
 
 // Factor the SPD tile D (lower triangle used; identity-padded) and write
-// L^-1 to Dinv (D is left as it is), in two warps of the CTA: lane i of warp
-// 0 keeps row i of the tile in registers, lane i of warp 1 column i of L^-1
-// (forward substitution against L).  Columns are factored two at a time:
-// every lane of warp 0 forms the 2x2 pivot block from three shuffles (both
-// reciprocal square roots issued together: the second pivot is det / p0),
-// then its own entries of both columns, which go to shared memory (col: two
-// buffers of two columns, piv: two buffers of the pivot block's r0, l10,
-// r1) for the trailing updates -- of the tile's rows in warp 0, of the
-// inverse's columns in warp 1, after one 64-thread named barrier per column
-// pair.  A buffer is rewritten two column pairs later, after warp 1 has
-// passed the next barrier, so one barrier per pair suffices.  No divisions.
-// Returns false (in warp 0) when a pivot was not positive.
-constexpr int kPotrfBarrier = 1;   // named barrier id (0 is __syncthreads)
+// L^-1 to Dinv and its rows, as they are found, to Lg (unless null); called by
+// the warps 0..3 of a CTA.  Columns are factored two at a time: the 2x2 pivot
+// block gives both reciprocal square roots together (the second pivot is
+// det / p0), no divisions.  Returns false (in one of the warps) when a pivot
+// was not positive.  The two precisions split the work differently, with the
+// same arithmetic per element.
+constexpr int kPotrfBarrier = 1;   // named barriers 1 and 2: FP64 tile factorization (0 is __syncthreads)
+constexpr int kQuadBarrier = 3;    // the four warps 0..3
+constexpr int kAuxBarrier = 4;     // the four warps 4..7
 
-__device__ __forceinline__ void potrf_pair_sync() {
-  asm volatile("bar.sync %0, 64;\n" ::"n"(kPotrfBarrier) : "memory");
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }
 
+// (one evaluation for both: an FP64 instruction costs the same for one lane)
+__device__ __forceinline__ void rsqrt_two(double a, double b, double& ra, double& rb) {
+  const double r = rsqrt((threadIdx.x & 1) ? b : a);
+  ra = __shfl_sync(0xffffffffu, r, 0);
+  rb = __shfl_sync(0xffffffffu, r, 1);
+}
+
+// Shared scratch of one tile factorization; `step` must be 0 before the first.
 template <typename T>
-__device__ bool pair_potrf_inverse(const Tile<T>& D, Tile<T>& Dinv, T* col, T* piv, int warp, int lane) {
-  using V = Vec16<T>;
-  constexpr int N = V::N;
+struct PotrfBuf;
+template <>
+struct PotrfBuf<double> {
+  double f[4][2][kTile];
+  int step;
+};
+template <>
+struct PotrfBuf<float> {
+  alignas(16) float f[kTile / 2][2][kTile];   // the columns of L, pair by pair
+  float4 piv[kTile / 2];                        // r0, l10, r1 of each pair
+  int step;                                     // pairs published so far
+};
+
+__device__ __forceinline__ void st_release_shared(int* p, int v) {
+  asm volatile("st.release.cta.shared::cta.u32 [%0], %1;\n" ::"r"(unsigned(__cvta_generic_to_shared(p))), "r"(v)
+               : "memory");
+}
+__device__ __forceinline__ int ld_acquire_shared(const int* p) {
+  int v;
+  asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];\n"
+               : "=r"(v)
+               : "r"(unsigned(__cvta_generic_to_shared(p)))
+               : "memory");
+  return v;
+}
+
+// FP32: latency, not throughput, so one warp runs the whole chain of pivots
+// without ever waiting for another: lane i of warp 0 keeps row i of the tile
+// in registers, lane i of warp 1 column i of L^-1 (forward substitution
+// against L), one step behind.  A step's critical part goes through
+// shuffles only: the next pair's two columns are updated and its pivot block
+// read first, the rest of the trailing updates (from the published columns,
+// four to a load) fills the latency of the next pivots' square roots.  Warp
+// 1 waits for `step`, which warp 0 always reaches (it has no wait of its
+// own; the limit only makes the bound explicit).  16 pairs in 1.0 us; with the tile's columns spread over four
+// warps and a barrier a pair (the FP64 form) 2.2 us.
+__device__ __forceinline__ bool tile_potrf_inverse(const Tile<float>& D, Tile<float>& Dinv, PotrfBuf<float>& fb,
+                                                   float* __restrict__ Lg, int warp, int lane) {
   constexpr unsigned FULL = 0xffffffffu;
   bool ok = true;
   if (warp == 0) {
-    T a[kTile];
+    float a[kTile];
 #pragma unroll
-    for (int q = 0; q < kTile; q += N) V::unpack(*reinterpret_cast<const typename V::V*>(&D[lane][q]), a + q);
+    for (int q = 0; q < kTile; q += 4) load16(&D[lane][q], a + q);
+    float p0 = __shfl_sync(FULL, a[0], 0), p1 = __shfl_sync(FULL, a[0], 1), p2 = __shfl_sync(FULL, a[1], 1);
     // j is a compile-time constant in every step, so a[] stays in registers
-    static_for<0, kTile, 2>([&](auto jc) {
-      constexpr int j = decltype(jc)::value;
-      const T p0 = __shfl_sync(FULL, a[j], j);
-      const T p1 = __shfl_sync(FULL, a[j], j + 1);
-      const T p2 = __shfl_sync(FULL, a[j + 1], j + 1);
+    static_for<0, kTile / 2, 1>([&](auto sc) {
+      constexpr int s = decltype(sc)::value, j = 2 * s;
+      const float det = fmaf(p0, p2, -(p1 * p1));
+      const float r0 = rsqrtf(p0), rd = rsqrtf(det);
+      const float l00 = p0 * r0;             // sqrt(p0)
+      const float l10 = p1 * r0;
+      const float r1 = l00 * rd;             // 1 / sqrt(det / p0)
+      ok = ok && (p0 > 0.0f) && (det > 0.0f);
+      // rows above the pair hold nothing here; the pair's own rows are not
+      // read by the trailing updates, which start below them
+      const float li0 = lane > j ? a[j] * r0 : 0.0f;
+      const float li1 = lane > j + 1 ? fmaf(-li0, l10, a[j + 1]) * r1 : 0.0f;
+      fb.f[s][0][lane] = li0;
+      fb.f[s][1][lane] = li1;
+      if (lane == 0) fb.piv[s] = make_float4(r0, l10, r1, 0.0f);
+      if constexpr (j + 2 < kTile) {
+        const float c00 = __shfl_sync(FULL, li0, j + 2), c10 = __shfl_sync(FULL, li1, j + 2);
+        const float c01 = __shfl_sync(FULL, li0, j + 3), c11 = __shfl_sync(FULL, li1, j + 3);
+        a[j + 2] = fmaf(-li1, c10, fmaf(-li0, c00, a[j + 2]));
+        a[j + 3] = fmaf(-li1, c11, fmaf(-li0, c01, a[j + 3]));
+        p0 = __shfl_sync(FULL, a[j + 2], j + 2);
+        p1 = __shfl_sync(FULL, a[j + 2], j + 3);
+        p2 = __shfl_sync(FULL, a[j + 3], j + 3);
+      }
+      __syncwarp();
+      if (lane == 0) st_release_shared(&fb.step, s + 1);
+#pragma unroll
+      for (int l = (j + 4) / 4 * 4; l < kTile; l += 4) {
+        float c0[4], c1[4];
+        load16(&fb.f[s][0][l], c0);
+        load16(&fb.f[s][1][l], c1);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (l + e >= j + 4) a[l + e] = fmaf(-li1, c1[e], fmaf(-li0, c0[e], a[l + e]));
+      }
+    });
+  } else if (warp == 1) {
+    float x[kTile];
+#pragma unroll
+    for (int r = 0; r < kTile; ++r) x[r] = (r == lane) ? 1.0f : 0.0f;
+    static_for<0, kTile / 2, 1>([&](auto sc) {
+      constexpr int s = decltype(sc)::value, j = 2 * s;
+      for (int spin = 0; ld_acquire_shared(&fb.step) <= s && ok; ++spin) ok = spin < (1 << 20);
+      const float4 pv = fb.piv[s];   // r0, l10, r1
+      x[j] *= pv.x;
+      x[j + 1] = fmaf(-pv.y, x[j], x[j + 1]) * pv.z;
+      Dinv[j][lane] = x[j];
+      Dinv[j + 1][lane] = x[j + 1];
+      if (Lg) {
+        Lg[j * kTile + lane] = x[j];
+        Lg[(j + 1) * kTile + lane] = x[j + 1];
+      }
+#pragma unroll
+      for (int l = (j + 2) / 4 * 4; l < kTile; l += 4) {
+        float c0[4], c1[4];
+        load16(&fb.f[s][0][l], c0);
+        load16(&fb.f[s][1][l], c1);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (l + e >= j + 2) x[l + e] = fmaf(-c1[e], x[j + 1], fmaf(-c0[e], x[j], x[l + e]));
+      }
+    });
+    __syncwarp();
+    if (lane == 0) fb.step = 0;   // warp 0 has published its last pair
+  }
+  return ok;
+}
+
+// FP64: bound by its pipe (64 cycles an instruction and warp, whatever the
+// lanes), so the work is spread over the four schedulers: the pair s =
+// (2s, 2s + 1) belongs to warp s mod 4, lane t of which holds, for each of its
+// columns l, the tile's entry (t, l) for t >= l and the inverse's entry (l, t)
+// for t < l: a step's updates of both are the same FMAs with the step's two
+// column vectors, so one instruction serves a column of the tile and a row of
+// the inverse.  The pair's owner scales its two columns, publishes them (four
+// buffers of two columns) and arrives at the step's barrier without waiting;
+// the next pair's owner updates that pair first and publishes it before it
+// catches up with its other columns.
+__device__ __forceinline__ bool tile_potrf_inverse(const Tile<double>& D, Tile<double>& Dinv, PotrfBuf<double>& fb,
+                                                   double* __restrict__ Lg, int warp, int lane) {
+  using T = double;
+  constexpr unsigned FULL = 0xffffffffu;
+  bool ok = true;
+  T v[8];   // columns 2 (warp + 4 p) + h at v[2 p + h]
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int l = 2 * (warp + 4 * p) + h;
+      v[2 * p + h] = lane >= l ? D[lane][l] : T(0);
+    }
+  // step s's update of the warp's pair p
+  auto update = [&](auto sc, auto pc) {
+    constexpr int s = decltype(sc)::value, p = decltype(pc)::value;
+    const T* f0 = fb.f[s & 3][0];
+    const T* f1 = fb.f[s & 3][1];
+    const int l = 2 * (warp + 4 * p);
+    const T g0 = f0[lane], g1 = f1[lane];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const T c0 = f0[l + h], c1 = f1[l + h];
+      const T a = fma(-g1, c1, fma(-g0, c0, v[2 * p + h]));
+      if (lane >= l + h || lane <= 2 * s + 1) v[2 * p + h] = a;
+    }
+  };
+  static_for<0, kTile / 2, 1>([&](auto sc) {
+    constexpr int s = decltype(sc)::value, j = 2 * s, p = s >> 2;
+    if (warp == (s & 3)) {   // the pair's owner: pivot, columns, publication
+      const T a0 = v[2 * p], a1 = v[2 * p + 1];
+      const T p0 = __shfl_sync(FULL, a0, j);
+      const T p1 = __shfl_sync(FULL, a0, j + 1);
+      const T p2 = __shfl_sync(FULL, a1, j + 1);
       const T det = fma(p0, p2, -(p1 * p1));
-      const T r0 = rsqrt(p0);
-      const T rd = rsqrt(det);
+      T r0, rd;
+      rsqrt_two(p0, det, r0, rd);
       const T l00 = p0 * r0;             // sqrt(p0)
       const T l10 = p1 * r0;
       const T r1 = l00 * rd;             // 1 / sqrt(det / p0)
-      const T l11 = det * rd * r0;       // sqrt(det / p0)
       ok = ok && (p0 > T(0)) && (det > T(0));
-      const T li0 = (lane > j) ? a[j] * r0 : ((lane == j) ? l00 : T(0));
-      const T li1 = (lane > j + 1) ? fma(-li0, l10, a[j + 1]) * r1 : ((lane == j + 1) ? l11 : T(0));
-      a[j] = li0;
-      a[j + 1] = li1;
-      const int buf = (j >> 1) & 1;
-      T* cb = col + buf * 2 * kTile;
-      cb[lane] = li0;
-      cb[kTile + lane] = li1;
-      if (lane == 0) {
-        piv[4 * buf] = r0;
-        piv[4 * buf + 1] = l10;
-        piv[4 * buf + 2] = r1;
+      const T f0 = lane == j ? r0 : a0 * r0;
+      const T f1 = lane == j + 1 ? r1 : fma(-f0, l10, a1) * r1;
+      fb.f[s & 3][0][lane] = lane == j + 1 ? T(0) : f0;   // (row j of the inverse ends at j)
+      fb.f[s & 3][1][lane] = f1;
+      bar_arrive(kPotrfBarrier + (s & 1), 128);
+      const T x0 = lane <= j ? f0 : T(0), x1 = lane <= j + 1 ? f1 : T(0);
+      Dinv[j][lane] = x0;
+      Dinv[j + 1][lane] = x1;
+      if (Lg) {
+        Lg[j * kTile + lane] = x0;
+        Lg[(j + 1) * kTile + lane] = x1;
       }
-      potrf_pair_sync();
-#pragma unroll
-      for (int l = j + 2; l < kTile; ++l) {
-        const T c0 = cb[l], c1 = cb[kTile + l];
-        a[l] = fma(-li0, c0, a[l]);
-        a[l] = fma(-li1, c1, a[l]);
+      __syncwarp();
+      // the other pairs: step s - 1 (left out below), then this step
+      static_for<p + 1, 4, 1>([&](auto pc) {
+        if constexpr (s > 0) update(std::integral_constant<int, (s > 0 ? s - 1 : 0)>{}, pc);
+        update(sc, pc);
+      });
+    } else {
+      bar_sync(kPotrfBarrier + (s & 1), 128);
+      if (s + 1 < kTile / 2 && warp == ((s + 1) & 3)) {   // next: its pivot pair only
+        constexpr int pn = s + 1 < kTile / 2 ? (s + 1) >> 2 : 3;
+        update(sc, std::integral_constant<int, pn>{});
+      } else {
+        static_for<p, 4, 1>([&](auto pc) {
+          constexpr int pp = decltype(pc)::value;
+          if (pp > p || warp > (s & 3)) update(sc, pc);
+        });
       }
-    });
-  } else {
-    T x[kTile];
-#pragma unroll
-    for (int r = 0; r < kTile; ++r) x[r] = (r == lane) ? T(1) : T(0);
-    static_for<0, kTile, 2>([&](auto jc) {
-      constexpr int j = decltype(jc)::value;
-      potrf_pair_sync();
-      const int buf = (j >> 1) & 1;
-      const T* cb = col + buf * 2 * kTile;
-      const T r0 = piv[4 * buf], l10 = piv[4 * buf + 1], r1 = piv[4 * buf + 2];
-      x[j] *= r0;
-      x[j + 1] = fma(-l10, x[j], x[j + 1]) * r1;
-#pragma unroll
-      for (int l = j + 2; l < kTile; ++l) {
-        const T c0 = cb[l], c1 = cb[kTile + l];
-        x[l] = fma(-c0, x[j], x[l]);
-        x[l] = fma(-c1, x[j + 1], x[l]);
-      }
-    });
-#pragma unroll
-    for (int r = 0; r < kTile; ++r) Dinv[r][lane] = x[r];
-  }
+    }
+  });
   return ok;
 }
 
@@ -2109,8 +2360,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_chol_step(DevPl
   if (need_d) fd.store(D);
   __syncthreads();
   if (k >= 0) {
-    tile_sub_xyt<T>(A, Li, Lj);
-    if (j == c && i != c) tile_sub_xyt<T>(D, Lj, Lj);
+    if (i == j) tile_sub_sym(A, Li); else tile_sub_xyt<T>(A, Li, Lj);
+    if (j == c && i != c) tile_sub_sym(D, Lj);
   }
   if (j == c && tid < kTile) {
     // b_i after column k: b_i - L_ik y_k
@@ -2132,10 +2383,15 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_chol_step(DevPl
   }
   // column c: factor the diagonal tile (own tile when i == c)
   __shared__ int ok_s;
-  __shared__ T colbuf[4 * kTile + 8];
-  if (warp < 2) {
-    const bool ok = pair_potrf_inverse<T>(i == c ? A : D, Dinv, colbuf, colbuf + 4 * kTile, warp, lane);
-    if (warp == 0 && lane == 0) ok_s = ok ? 1 : 0;
+  __shared__ PotrfBuf<T> fb;
+  if (tid == 0) {
+    ok_s = 1;
+    fb.step = 0;
+  }
+  __syncthreads();
+  if (warp < 4) {
+    T* Lg = i == c ? tptr_mut<T>(d.Linv) + ((long long)p * d.max_nt + c) * kTile * kTile : nullptr;
+    if (!tile_potrf_inverse(i == c ? A : D, Dinv, fb, Lg, warp, lane) && lane == 0) ok_s = 0;
   }
   __syncthreads();
   if (!ok_s) {
@@ -2144,33 +2400,19 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_chol_step(DevPl
   }
   const int mi = tile_rows(n, i);
   if (i == c) {
-    T* Lg = tptr_mut<T>(d.Linv) + ((long long)p * d.max_nt + c) * kTile * kTile;
-    for (int e = tid; e < kTile * kTile; e += blockDim.x) Lg[e] = Dinv[e / kTile][e % kTile];
-    if (tid < kTile) {
+    if (tid < mi) {
       T y = T(0);
 #pragma unroll 8
       for (int q = 0; q < kTile; ++q) y += Dinv[tid][q] * tv[q];
-      yk[tid] = y;
+      b[kTile * c + tid] = y;
     }
-    __syncthreads();
-    if (tid < mi) b[kTile * c + tid] = yk[tid];
     return;
   }
   // i > c: L_ic = A_ic L_cc^-T, and the column-k part of the forward solve
   if (tid < mi) b[kTile * i + tid] = tv[tid];
-  if (tid < 128) {
-    T sv[8];
-    tile_xyt<T>(A, Dinv, sv);
-    const int r = tid >> 3, c0 = tid & 7;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (r + 16 * h < mi) {
-        T* row = S + (long long)(kTile * i + r + 16 * h) * n + kTile * c;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) row[c0 + 8 * u] = sv[4 * h + u];
-      }
-    }
-  }
+  tile_panel<T, 8>(A, Dinv, Li, warp, lane);   // (Li is free again)
+  __syncthreads();
+  for (int r = warp; r < mi; r += 8) S[(long long)(kTile * i + r) * n + kTile * c + lane] = Li[r][lane];
 }
 
 // Dataflow factorization of one problem's reduced system in a single
@@ -2183,20 +2425,49 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_chol_step(DevPl
 // forward solve y_j = L_jj^-1 b_j) or its panel L_ij = A_ij L_jj^-T.  A
 // finished factor or panel is written to global memory (L into S, L_jj^-1
 // into Linv, y_j into b) and announced by storing the launch's epoch into
-// the tile's flag with release semantics; consumers poll flags with acquire
-// loads and read the data through L2.  Each CTA runs, among its tiles whose
-// next task has its inputs published, the one with the smallest (j, i), and
-// applies up to kDfBatch consecutive ready updates of that tile with all of
-// their loads in flight together.  Per element the arithmetic is exactly
-// that of k_chol_step (same tile routines, same order of updates), so both
-// schedules give the same bits.  Every wait is bounded: a CTA that sees
-// nothing ready for DevPlan::df_spin_limit polls records a timeout and leaves; a
-// failed pivot or a timeout raises the abort word, which every waiting CTA
-// checks.
+// the tile's flag with release semantics (y_j has its own, in the upper
+// triangle of the flags); consumers poll flags with acquire loads and read
+// the data through L2.  Each CTA runs, among its tiles whose next task has its
+// inputs published, the one with the smallest (j, i), and applies up to
+// df_batch consecutive ready updates of that tile with all of their loads in
+// flight together.  Per element the arithmetic is exactly that of k_chol_step
+// (same tile routines, same order of updates), so both schedules give the
+// same bits.
+//
+// The critical path is the chain L_jj^-1 -> panel (j+1, j) -> last update of
+// (j+1, j+1) -> its factor.  The chain task of a row does these in one go:
+// warps 0..3 take the update and the factor, warps 4..7 meanwhile publish
+// the panel (the next row's CTA then updates its own subdiagonal tile while
+// this row is factored) and bring b_i up to date.  The rows of L_jj^-1 are
+// stored as they are found, so the flag follows the last of them directly,
+// before y_j.  With at least two CTAs per tile row (DevPlan::df_rows), row i's
+// CTA owns nothing but the row's last tiles (df_row_tiles) and runs a fixed
+// program instead of the scheduler: the updates of all of them column by
+// column, then the panel (i, i-2) with its updates, then the chain task, so
+// that the row is always waiting for L_{i-1,i-1}^-1 when it comes.  Scheduled
+// tile by tile, every second row was late for it by an update of its
+// diagonal tile and ran its panel, that update and its factor as three tasks
+// (7.5 us a row instead of 4.1).  With three CTAs per row (FP32), a second CTA
+// keeps the three columns left of those in the same way (df_helpers): panels
+// that wait their turn in a worker's queue are then needed several chain steps
+// later instead of one.
+//
+// Every wait is bounded: a CTA that sees nothing ready for
+// DevPlan::df_spin_limit polls records a timeout and leaves; a failed pivot
+// or a timeout raises the abort word, which every waiting CTA checks.
 constexpr int kDfThreads = 256;
 
 template <typename T>
 __host__ __device__ constexpr int df_batch() { return 2; }
+
+// Tiles of row i kept by its own CTA: (i, i), (i, i-1) and, in FP32, (i, i-2).
+// An FP64 update takes 8 us of one SM's FP64 pipe, so a third tile would make
+// the row's updates slower than the chain they have to keep ahead of.
+template <typename T>
+__host__ __device__ constexpr int df_row_tiles() { return sizeof(T) == 4 ? 3 : 2; }
+// Tiles kept by row i's second CTA, left of those.
+template <typename T>
+__host__ __device__ constexpr int df_helper_tiles() { return sizeof(T) == 4 ? 3 : 0; }
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -2207,6 +2478,13 @@ __device__ __forceinline__ unsigned long long global_ns() {
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// A relaxed poll: several of one thread are in flight together (acquire loads
+// wait for one another); a fence must follow before the data is read.
+__device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
@@ -2224,6 +2502,43 @@ __device__ __forceinline__ void fetch_rect_cg(TileFetch<T>& f, const T* S, int n
   }
 }
 
+// The tile (ti, tj) left of the diagonal (all 32 columns) through L2 by the
+// threads t = 0 .. 127 of a thread group.
+template <typename T>
+struct HalfFetch {
+  T v[kTile * kTile / 128];
+  __device__ __forceinline__ void load(const T* S, int n, int ti, int tj, int t) {
+    const int mi = tile_rows(n, ti), r0 = t >> 5, c = t & 31;
+    const T* p = S + (long long)(kTile * ti + r0) * n + kTile * tj + c;
+#pragma unroll
+    for (int u = 0; u < kTile / 4; ++u) v[u] = r0 + 4 * u < mi ? __ldcg(p + (long long)(4 * u) * n) : T(0);
+  }
+  __device__ __forceinline__ void store(Tile<T>& tile, int t) const {
+#pragma unroll
+    for (int u = 0; u < kTile / 4; ++u) tile[(t >> 5) + 4 * u][t & 31] = v[u];
+  }
+};
+
+// A contiguous 32x32 tile (an L_jj^-1) through L2, 16 bytes a load, by the
+// threads t = 0 .. kThreads - 1 of a thread group.
+template <typename T, int kThreads>
+struct InvFetch {
+  static constexpr int N = Vec16<T>::N, kVecs = kTile * kTile / N / kThreads;
+  typename Vec16<T>::V v[kVecs];
+  __device__ __forceinline__ void load(const T* Li, int t) {
+#pragma unroll
+    for (int u = 0; u < kVecs; ++u)
+      v[u] = __ldcg(reinterpret_cast<const typename Vec16<T>::V*>(Li) + t + u * kThreads);
+  }
+  __device__ __forceinline__ void store(Tile<T>& tile, int t) const {
+#pragma unroll
+    for (int u = 0; u < kVecs; ++u) {
+      const int e = (t + u * kThreads) * N;
+      *reinterpret_cast<typename Vec16<T>::V*>(&tile[e / kTile][e % kTile]) = v[u];
+    }
+  }
+};
+
 template <typename T>
 size_t df_smem_bytes(int max_own) {
   return sizeof(Tile<T>) * size_t(max_own + 2 * df_batch<T>() + 1) +
@@ -2233,9 +2548,10 @@ size_t df_smem_bytes(int max_own) {
 template <typename T>
 __global__ void __launch_bounds__(kDfThreads, 1) k_chol_dataflow(DevPlan d) {
   constexpr int NB = df_batch<T>();
-  enum { kIdle = 0, kUpdate = 1, kFinish = 2, kChain = 3, kExit = 4, kChain2 = 5 };
+  enum { kIdle = 0, kUpdate = 1, kFinish = 2, kChain = 3, kExit = 4 };
   extern __shared__ __align__(16) unsigned char df_raw[];
-  __shared__ T yv[NB][kTile], colbuf[4 * kTile + 8];
+  __shared__ T yv[NB][kTile];
+  __shared__ PotrfBuf<T> fb;
   __shared__ int s_sel, s_cnt, s_mode, s_ok;
   const int p = 0;
   const ProbInfo pi = d.prob[p];
@@ -2258,38 +2574,395 @@ __global__ void __launch_bounds__(kDfThreads, 1) k_chol_dataflow(DevPlan d) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned epoch = *reinterpret_cast<volatile unsigned*>(d.df_sync) + 1u;
 
-  // factor the diagonal tile A[t] of row i in warp 0 and publish L_ii^-1 and
-  // y_i = L_ii^-1 b_i; false (after raising the abort word) on a bad pivot
+  // optional timeline (thread 0): per task its wait start, selection, end
+  unsigned long long* tr = d.df_trace ? d.df_trace + size_t(blockIdx.x) * kDfTraceCap * 4 : nullptr;
+  // y_k's flag (row 0 of the upper triangle; nobody waits for the last y)
+  auto y_flag = [&](int kk) { return flags + kk + 1; };
+  // L_ii^-1 of row i is out (warps 0..3 stored its rows): announce it, then
+  // form and announce y_i = L_ii^-1 b_i; false (after raising the abort word)
+  // on a bad pivot
   auto finish_diag = [&](int t, int i) -> bool {
-    if (warp < 2) {
-      const bool ok = pair_potrf_inverse<T>(A[t], Dinv, colbuf, colbuf + 4 * kTile, warp, lane);
-      if (warp == 0 && lane == 0) s_ok = ok ? 1 : 0;
-    }
     __syncthreads();
-    if (!s_ok) {
-      if (tid == 0) {
+    if (s_ok <= 0) {
+      if (tid == 0 && s_ok == 0) {
         d.factor_flag[p] = 1;
         __threadfence();
         atomicExch(d.df_sync + 2, epoch);
       }
       return false;
     }
-    T* Lo = Lg + (long long)i * kTile * kTile;
-    for (int e = tid; e < kTile * kTile; e += blockDim.x) Lo[e] = Dinv[e / kTile][e % kTile];
-    if (tid < kTile) {
+    if (tid == 0) st_release_u32(flags + (long long)i * nt + i, epoch);
+    if (warp == 1) {
       T y = T(0);
 #pragma unroll 8
-      for (int q = 0; q < kTile; ++q) y += Dinv[tid][q] * bown[t * kTile + q];
-      if (tid < tile_rows(n, i)) b[kTile * i + tid] = y;
+      for (int q = 0; q < kTile; ++q) y += Dinv[lane][q] * bown[t * kTile + q];
+      if (lane < tile_rows(n, i)) b[kTile * i + lane] = y;
+      __syncwarp();
+      if (lane == 0 && i + 1 < nt) st_release_u32(y_flag(i), epoch);
     }
-    __syncthreads();
-    if (tid == 0) {
-      st_release_u32(flags + (long long)i * nt + i, epoch);
-      kt_s[t] = i + 1;
-    }
+    if (tid == 0) kt_s[t] = i + 1;
     return true;
   };
 
+  // W[0] = the panel L_ij = A_ij L_jj^-T (L_jj^-1 is published); ends with a barrier
+  auto panel_of = [&](const Tile<T>& Aij, int j) {
+    InvFetch<T, kDfThreads> f;
+    f.load(Lg + (long long)j * kTile * kTile, tid);
+    f.store(Dinv, tid);
+    __syncthreads();
+    tile_panel<T, 8>(Aij, Dinv, W[0], warp, lane);
+    __syncthreads();
+  };
+  // the rows of the panel W[0] into S, by `warps` warps (this one is the w-th)
+  auto publish_panel = [&](int i, int j, int w, int warps) {
+    const int mi = tile_rows(n, i);
+    T* const Sij = S + (long long)kTile * i * n + kTile * j;
+    for (int r = w; r < mi; r += warps) Sij[(long long)r * n + lane] = W[0][r][lane];
+  };
+  // one warp waits for the flags f[0 .. cnt) (one per lane; null: none);
+  // false when the launch is aborted or the limit ran out
+  auto wait_flag = [&](const unsigned* f) -> bool {
+    long long spin = 0;
+    for (;;) {
+      if (__all_sync(0xffffffffu, f == nullptr || ld_acquire_u32(f) == epoch)) return true;
+      ++spin;
+      int stop = 0;
+      if (lane == 0 && (spin & 15) == 0) stop = ld_acquire_u32(d.df_sync + 2) == epoch;
+      if (lane == 0 && !stop && spin > d.df_spin_limit) {
+        d.factor_flag[p] = 2;   // timed out
+        __threadfence();
+        atomicExch(d.df_sync + 2, epoch);
+        stop = 1;
+      }
+      if (__shfl_sync(0xffffffffu, stop, 0)) return false;
+    }
+  };
+  // bown[t] -= L yv[0] for a tile L of row i (one warp)
+  auto rhs_sub = [&](int t, const Tile<T>& L) {
+    T tv = bown[t * kTile + lane];
+#pragma unroll 8
+    for (int q = 0; q < kTile; ++q) tv -= L[lane][q] * yv[0][q];
+    bown[t * kTile + lane] = tv;
+  };
+  // bown[t] -= L y_k once y_k is out (one warp); false when aborted
+  auto row_rhs = [&](int t, const Tile<T>& L, int kk) -> bool {
+    if (!wait_flag(lane == 0 ? y_flag(kk) : nullptr)) return false;
+    yv[0][lane] = __ldcg(b + kTile * kk + lane);
+    __syncwarp();
+    rhs_sub(t, L);
+    __syncwarp();
+    return true;
+  };
+  // the chain task of row i (tile t = (i, i-1), td = (i, i)); false when it
+  // failed or the launch is aborted
+  auto chain_task = [&](int t, int td, int i) -> bool {
+    const int j = i - 1;
+    panel_of(A[t], j);
+    if (warp < 4) {
+      tile_sub_sym(A[td], W[0]);
+      bar_sync(kQuadBarrier, 128);
+      if (!tile_potrf_inverse(A[td], Dinv, fb, Lg + (long long)i * kTile * kTile, warp, lane) && lane == 0)
+        s_ok = 0;
+    } else {
+      publish_panel(i, j, warp - 4, 4);
+      bar_sync(kAuxBarrier, 128);
+      if (tid == 128) st_release_u32(flags + (long long)i * nt + j, epoch);
+      if (warp == 5 && !row_rhs(td, W[0], j) && lane == 0) s_ok = -1;
+    }
+    return finish_diag(td, i);
+  };
+  // every thread waits while warp 0 polls (one flag per lane)
+  auto cta_wait = [&](const unsigned* f) -> bool {
+    if (warp == 0) {
+      const bool ok = wait_flag(f);
+      if (lane == 0) s_mode = ok ? 1 : 0;
+    }
+    __syncthreads();
+    const bool ok = s_mode != 0;
+    __syncthreads();
+    return ok;
+  };
+  // the fixed program of row i's own CTA: its tiles are (i, i-2), (i, i-1),
+  // (i, i) (the last `nown` of them).  The chain task runs once per CTA, so its
+  // instructions would come from L2 while every later row waits: it is run
+  // through once on scratch tiles first, from the same code.
+  int rp_n = 0;
+  unsigned long long rp_wait = 0, rp_sel = 0;
+  auto note_wait = [&] { if (tr && tid == 0) rp_wait = global_ns(); };
+  auto note_start = [&] { if (tr && tid == 0) rp_sel = global_ns(); };
+  auto note_end = [&](int mode, int j, int kk) {
+    if (!tr || tid != 0 || rp_n >= kDfTraceCap) return;
+    unsigned long long* e = tr + 4 * rp_n++;
+    e[0] = (unsigned long long)mode << 56 | (unsigned long long)blockIdx.x << 40 | (unsigned long long)j << 24 |
+           (unsigned long long)kk << 8 | 1ull;
+    e[1] = rp_wait;
+    e[2] = rp_sel;
+    e[3] = global_ns();
+  };
+  auto row_chain = [&](int i, int t1, int td, bool real) {
+    if (i > 0) {
+      if (real) {
+        panel_of(A[t1], i - 1);
+      } else {
+        tile_panel<T, 8>(W[1], W[2], W[0], warp, lane);
+        __syncthreads();
+      }
+    }
+    if (warp < 4) {
+      Tile<T>& Di = real ? A[td] : W[3];
+      if (i > 0) tile_sub_sym(Di, W[0]);
+      bar_sync(kQuadBarrier, 128);
+      if (!tile_potrf_inverse(Di, Dinv, fb, real ? Lg + (long long)i * kTile * kTile : nullptr, warp, lane) &&
+          lane == 0 && real)
+        s_ok = 0;
+    } else if (i > 0 && real) {
+      publish_panel(i, i - 1, warp - 4, 4);
+      bar_sync(kAuxBarrier, 128);
+      if (tid == 128) st_release_u32(flags + (long long)i * nt + i - 1, epoch);
+      if (warp == 5 && !row_rhs(td, W[0], i - 1) && lane == 0) s_ok = -1;
+    }
+    if (real)
+      finish_diag(td, i);
+    else
+      __syncthreads();
+  };
+  auto row_steps = [&](int i) -> bool {
+    const int td = nown - 1, t1 = nown - 2, t2 = nown - 3;   // (negative: none)
+    const int steps = t2 >= 0 ? i - 2 : i - 1;
+    for (int kk = 0; kk < steps; ++kk) {   // column kk into every tile of the row
+      note_wait();
+      const unsigned* f = nullptr;
+      if (lane == 0) f = flags + (long long)i * nt + kk;
+      if (lane == 1) f = flags + (long long)(i - 1) * nt + kk;
+      if (lane == 2 && t2 >= 0) f = flags + (long long)(i - 2) * nt + kk;
+      if (lane == 3) f = y_flag(kk);
+      if (!cta_wait(f)) return false;
+      note_start();
+      {
+        TileFetch<T> f0, f1, f2;
+        fetch_rect_cg<T>(f0, S, n, i, kk);
+        fetch_rect_cg<T>(f1, S, n, i - 1, kk);
+        if (t2 >= 0) fetch_rect_cg<T>(f2, S, n, i - 2, kk);
+        if (warp == 0) yv[0][lane] = __ldcg(b + kTile * kk + lane);
+        f0.store(W[0]);
+        f1.store(W[1]);
+        if (t2 >= 0) f2.store(W[2]);
+      }
+      __syncthreads();
+      if (t2 >= 0) {
+        tile_sub_xyt_t<T>(A[warp < 4 ? t2 : t1], W[0], W[warp < 4 ? 2 : 1], tid & 127);
+        tile_sub_sym_half(A[td], W[0]);
+      } else if (warp < 4) {
+        tile_sub_sym(A[td], W[0]);
+      } else {
+        tile_sub_xyt_t<T>(A[t1], W[0], W[1], tid - 128);
+      }
+      if (warp == 7) rhs_sub(td, W[0]);
+      __syncthreads();
+      note_end(kUpdate, i, kk);
+    }
+    if (t2 >= 0) {   // the panel (i, i-2), then its column into the other two
+      const int j = i - 2;
+      note_wait();
+      if (!cta_wait(lane == 0 ? flags + (long long)j * nt + j : nullptr)) return false;
+      note_start();
+      panel_of(A[t2], j);
+      bool ok = true;
+      if (warp < 4) {
+        tile_sub_sym(A[td], W[0]);
+      } else {
+        publish_panel(i, j, warp - 4, 4);
+        bar_sync(kAuxBarrier, 128);
+        if (tid == 128) st_release_u32(flags + (long long)i * nt + j, epoch);
+        if (warp == 5) ok = row_rhs(td, W[0], j);
+        if (warp == 6) ok = wait_flag(lane == 0 ? flags + (long long)(i - 1) * nt + j : nullptr);
+      }
+      if (!ok && lane == 0) s_ok = -1;
+      __syncthreads();
+      if (s_ok < 0) return false;
+      TileFetch<T> f1;
+      fetch_rect_cg<T>(f1, S, n, i - 1, j);
+      f1.store(W[1]);
+      __syncthreads();
+      tile_sub_xyt<T>(A[t1], W[0], W[1]);
+      __syncthreads();
+      note_end(kFinish, j, j);
+    }
+    note_wait();
+    if (t1 >= 0 && !cta_wait(lane == 0 ? flags + (long long)(i - 1) * nt + i - 1 : nullptr)) return false;
+    note_start();
+    return true;
+  };
+  // the program of row i's second CTA (DevPlan::df_helpers): its tiles are
+  // the (up to three) columns left of the first CTA's, c0 .. c0 + nown - 1,
+  // updated together column by column, then their panels in order, each
+  // taken into the tiles right of it as soon as it is out
+  auto helper_program = [&](int i) -> bool {
+    const int c0 = i - 2 - nown;
+    for (int kk = 0; kk < c0; ++kk) {
+      const unsigned* f = nullptr;
+      if (lane == 0) f = flags + (long long)i * nt + kk;
+      if (lane >= 1 && lane <= nown) f = flags + (long long)(c0 + lane - 1) * nt + kk;
+      if (!cta_wait(f)) return false;
+      {
+        TileFetch<T> f0, f1, f2, f3;
+        fetch_rect_cg<T>(f0, S, n, i, kk);
+        fetch_rect_cg<T>(f1, S, n, c0, kk);
+        if (nown > 1) fetch_rect_cg<T>(f2, S, n, c0 + 1, kk);
+        if (nown > 2) fetch_rect_cg<T>(f3, S, n, c0 + 2, kk);
+        f0.store(W[0]);
+        f1.store(W[1]);
+        if (nown > 1) f2.store(W[2]);
+        if (nown > 2) f3.store(W[3]);
+      }
+      __syncthreads();
+      for (int t = tid >> 7; t < nown; t += 2) tile_sub_xyt_t<T>(A[t], W[0], W[1 + t], tid & 127);
+      __syncthreads();
+    }
+    for (int u = 0; u < nown; ++u) {
+      const int j = c0 + u;
+      if (!cta_wait(lane == 0 ? flags + (long long)j * nt + j : nullptr)) return false;
+      panel_of(A[u], j);
+      publish_panel(i, j, warp, 8);
+      __syncthreads();
+      if (tid == 128) st_release_u32(flags + (long long)i * nt + j, epoch);
+      if (u + 1 < nown) {
+        const int m = nown - u - 1;   // tiles right of it
+        if (!cta_wait(lane >= 1 && lane <= m ? flags + (long long)(j + lane) * nt + j : nullptr)) return false;
+        TileFetch<T> f1, f2;
+        fetch_rect_cg<T>(f1, S, n, j + 1, j);
+        if (m > 1) fetch_rect_cg<T>(f2, S, n, j + 2, j);
+        f1.store(W[1]);
+        if (m > 1) f2.store(W[2]);
+        __syncthreads();
+        const int t = tid >> 7;
+        if (t < m) tile_sub_xyt_t<T>(A[u + 1 + t], W[0], W[1 + t], tid & 127);
+        __syncthreads();
+      }
+    }
+    return true;
+  };
+  // a worker CTA beside row CTAs (df_rows): its two halves of four warps are
+  // workers of their own, half g with the tiles t = g (mod 2), so that one's
+  // loads and waits overlap the other's products.  Lane m of the half's first
+  // warp keeps its m-th tile's state (at most 32 tiles) and polls its flags;
+  // the ready tile with the smallest (j, i) is taken, up to four updates at a
+  // time with the next one's loads in flight, or its panel.
+  auto worker_program = [&] {
+    const int g = tid >> 7, gt = tid & 127, gw = warp & 3, bar = kQuadBarrier + g;
+    Tile<T>& X = W[2 * g];
+    Tile<T>& Y = W[2 * g + 1];
+    __shared__ int4 s_task[2];   // (tile, first column, count or 0: panel, 0 leave / 1 go / 2 wait)
+    int my_t = -1, my_i = 0, my_j = 0, my_k = 0;
+    if (gw == 0 && 2 * lane + g < nown) {
+      my_t = 2 * lane + g;
+      my_i = ti_s[my_t];
+      my_j = tj_s[my_t];
+    }
+    int left = (nown - g + 1) / 2, rp_n = 0;
+    long long spin = 0;
+    unsigned long long t_wait = 0, t_sel = 0;
+    if (tr && gt == 0) t_wait = global_ns();
+    while (left > 0) {
+      if (gw == 0) {
+        int c = 0, ready = 0;   // c updates ready, or the panel
+        if (my_t >= 0 && my_k < my_j) {
+          unsigned fi[4], fj[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            fi[u] = my_k + u < my_j ? ld_relaxed_u32(flags + (long long)my_i * nt + my_k + u) : 0u;
+            fj[u] = my_k + u < my_j ? ld_relaxed_u32(flags + (long long)my_j * nt + my_k + u) : 0u;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (c == u && my_k + u < my_j && fi[u] == epoch && fj[u] == epoch) c = u + 1;
+          ready = c > 0;
+        } else if (my_t >= 0 && my_k == my_j) {
+          ready = ld_relaxed_u32(flags + (long long)my_j * nt + my_j) == epoch;
+        }
+        const unsigned any = __ballot_sync(0xffffffffu, ready);   // (lanes are in (j, i) order)
+        if (any != 0) {
+          if (lane == __ffs(any) - 1) {
+            __threadfence();   // acquire what the polled flags announce
+            s_task[g] = make_int4(my_t, my_k, c, 1);
+            my_k += c > 0 ? c : 1;
+          }
+        } else {
+          ++spin;
+          if (lane == 0) {
+            int go = 2;
+            if ((spin & 15) == 0 && ld_acquire_u32(d.df_sync + 2) == epoch) {
+              go = 0;
+            } else if (spin > d.df_spin_limit) {
+              d.factor_flag[p] = 2;   // timed out
+              __threadfence();
+              atomicExch(d.df_sync + 2, epoch);
+              go = 0;
+            }
+            s_task[g] = make_int4(0, 0, 0, go);
+          }
+        }
+      }
+      bar_sync(bar, 128);
+      const int4 task = s_task[g];
+      if (task.w == 0) return;
+      if (task.w == 2) {
+        bar_sync(bar, 128);
+        continue;
+      }
+      if (tr && gt == 0) t_sel = global_ns();
+      const int t = task.x, i = ti_s[t], j = tj_s[t];
+      if (task.z > 0) {
+        HalfFetch<T> fx, fy;
+        fx.load(S, n, i, task.y, gt);
+        fy.load(S, n, j, task.y, gt);
+        for (int u = 0; u < task.z; ++u) {
+          fx.store(X, gt);
+          fy.store(Y, gt);
+          bar_sync(bar, 128);
+          if (u + 1 < task.z) {
+            fx.load(S, n, i, task.y + u + 1, gt);
+            fy.load(S, n, j, task.y + u + 1, gt);
+          }
+          tile_sub_xyt_t<T>(A[t], X, Y, gt);
+          bar_sync(bar, 128);
+        }
+      } else {
+        InvFetch<T, 128> f;
+        f.load(Lg + (long long)j * kTile * kTile, gt);
+        f.store(X, gt);
+        bar_sync(bar, 128);
+        tile_panel<T, 4>(A[t], X, Y, gw, lane);
+        bar_sync(bar, 128);
+        const int mi = tile_rows(n, i);
+        T* const Sij = S + (long long)kTile * i * n + kTile * j;
+        for (int r = gw; r < mi; r += 4) Sij[(long long)r * n + lane] = Y[r][lane];
+        bar_sync(bar, 128);
+        if (gt == 96) st_release_u32(flags + (long long)i * nt + j, epoch);
+        --left;
+      }
+      if (tr && gt == 0 && rp_n < kDfTraceCap / 2) {
+        unsigned long long* e = tr + 4 * (2 * rp_n++ + g);
+        e[0] = (unsigned long long)(task.z > 0 ? kUpdate : kFinish) << 56 | (unsigned long long)i << 40 |
+               (unsigned long long)j << 24 | (unsigned long long)task.y << 8 | (unsigned long long)task.z;
+        e[1] = t_wait;
+        e[2] = t_sel;
+        e[3] = t_wait = global_ns();
+      }
+    }
+  };
+  auto row_program = [&](int i) {
+    for (int pass = i > 0 ? 0 : 1; pass < 2; ++pass) {   // (row 0 starts at once)
+      if (pass == 1 && !row_steps(i)) return;
+      row_chain(i, nown - 2, nown - 1, pass == 1);
+    }
+    note_end(kChain, i - 1, i - 1);
+  };
+
+  if (tid == 0) {
+    s_ok = 1;
+    fb.step = 0;
+  }
   const LMState& st = d.state[p];
   const bool run = st.active && !d.factor_flag[p];
   if (run) {
@@ -2307,19 +2980,34 @@ __global__ void __launch_bounds__(kDfThreads, 1) k_chol_dataflow(DevPlan d) {
           if (ti_s[u] == ti_s[t] && tj_s[u] == ti_s[t]) pr = u;
       pr_s[t] = pr;
     }
-    for (int t = 0; t < nown; ++t) {      // owned tiles and rhs
-      TileFetch<T> f;
-      const int i = ti_s[t], j = tj_s[t];
-      if (i == j) f.diag(S, n, i); else f.rect(S, n, i, j);
-      f.store(A[t]);
-      if (i == j && tid < kTile) bown[t * kTile + tid] = tid < tile_rows(n, i) ? b[kTile * i + tid] : T(0);
+    for (int t0 = 0; t0 < nown; t0 += 4) {      // owned tiles and rhs, four tiles in flight
+      TileFetch<T> f[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (t0 + u < nown) {
+          const int i = ti_s[t0 + u], j = tj_s[t0 + u];
+          if (i == j) f[u].diag(S, n, i); else f[u].rect(S, n, i, j);
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (t0 + u < nown) {
+          const int t = t0 + u, i = ti_s[t];
+          f[u].store(A[t]);
+          if (i == tj_s[t] && tid < kTile) bown[t * kTile + tid] = tid < tile_rows(n, i) ? b[kTile * i + tid] : T(0);
+        }
     }
   }
   __syncthreads();
-  int ndone = run ? 0 : nown;
+  const int bx = int(blockIdx.x);
+  const bool row_cta = bx < d.df_rows + d.df_helpers;
+  if (run && bx < d.df_rows)
+    row_program(bx);
+  else if (run && row_cta && nown > 0)
+    helper_program(bx - d.df_rows);
+  else if (run && d.df_rows > 0 && nown > 0)
+    worker_program();
+  int ndone = run && d.df_rows == 0 ? 0 : nown;   // (without row CTAs: the scheduler below)
   long long idle = 0;
-  // optional timeline (thread 0): per task its wait start, selection, end
-  unsigned long long* tr = d.df_trace ? d.df_trace + size_t(blockIdx.x) * kDfTraceCap * 4 : nullptr;
   unsigned long long tr_wait = 0, tr_sel = 0, tr_meta = 0;
   int tr_n = 0;
   bool tr_open = false;
@@ -2347,7 +3035,7 @@ __global__ void __launch_bounds__(kDfThreads, 1) k_chol_dataflow(DevPlan d) {
 #pragma unroll
         for (int u = 0; u < NB; ++u) {
           fi[u] = (k + u < j) ? ld_acquire_u32(flags + (long long)i * nt + k + u) : 0u;
-          fj[u] = (k + u < j && i != j) ? ld_acquire_u32(flags + (long long)j * nt + k + u) : epoch;
+          fj[u] = (k + u < j) ? ld_acquire_u32(i != j ? flags + (long long)j * nt + k + u : y_flag(k + u)) : epoch;
         }
 #pragma unroll
         for (int u = 0; u < NB; ++u)
@@ -2355,34 +3043,42 @@ __global__ void __launch_bounds__(kDfThreads, 1) k_chol_dataflow(DevPlan d) {
       } else if (k == j) {
         c = (i == j || ld_acquire_u32(flags + (long long)j * nt + j) == epoch) ? 1 : 0;
       }
-      // a subdiagonal tile one update short of its panel: is L_jj^-1 out too?
-      int linv = 0;
-      if (pr_s[t] >= 0 && k == j - 1) linv = ld_acquire_u32(flags + (long long)j * nt + j) == epoch;
-      rd_s[t] = c | linv << 8;
+      rd_s[t] = c;
     }
     __syncthreads();
     if (tid == 0) {
       int sel = -1, cnt = 0, mode = kIdle;
       for (int t = 0; t < nown; ++t) {
-        if ((rd_s[t] & 0xff) > 0) {
-          const bool diag_at = pr_s[t] >= 0 && kt_s[pr_s[t]] == ti_s[t] - 1;
-          // the chain's subdiagonal tile keeps its last update for the fused
-          // task (below) until L_jj^-1 is out and its diagonal tile has all
-          // other updates: run alone it would split the chain into three
-          // tasks on the critical path (the inputs it waits for never
-          // depend on this tile)
-          if (pr_s[t] >= 0 && kt_s[t] == tj_s[t] - 1 && (!(rd_s[t] >> 8) || !diag_at)) continue;
+        if (rd_s[t] > 0) {
           sel = t;
-          cnt = rd_s[t] & 0xff;
+          cnt = rd_s[t];
           mode = kt_s[t] < tj_s[t] ? kUpdate : kFinish;
-          if (mode == kFinish && diag_at) mode = kChain;
-          // the last update of a subdiagonal tile, its panel and the next
-          // diagonal factor in one task when L_jj^-1 is already out
-          if (mode == kUpdate && diag_at && kt_s[t] == tj_s[t] - 1 && (rd_s[t] >> 8)) mode = kChain2;
+          // a subdiagonal panel with its diagonal tile one update short
+          if (mode == kFinish && pr_s[t] >= 0 && kt_s[pr_s[t]] == ti_s[t] - 1) mode = kChain;
           break;
         }
       }
-      if (sel < 0) {
+      // nothing left but the chain task: wait here for the one flag it
+      // needs, with the bounds of the general loop
+      if (sel < 0 && nown - ndone == 2) {
+        for (int t = 0; t < nown; ++t)
+          if (pr_s[t] >= 0 && kt_s[t] == tj_s[t] && kt_s[pr_s[t]] == ti_s[t] - 1) {
+            const unsigned* fl = flags + (long long)tj_s[t] * nt + tj_s[t];
+            while (idle <= d.df_spin_limit) {
+              if (ld_acquire_u32(fl) == epoch) {
+                sel = t;
+                cnt = 1;
+                mode = kChain;
+                break;
+              }
+              if ((++idle & 15) == 0 && ld_acquire_u32(d.df_sync + 2) == epoch) {
+                mode = kExit;
+                break;
+              }
+            }
+          }
+      }
+      if (sel < 0 && mode != kExit) {
         // the abort word is read every 16th idle round, the limit counted always
         if ((++idle & 15) == 0 && ld_acquire_u32(d.df_sync + 2) == epoch) {
           mode = kExit;
@@ -2431,7 +3127,7 @@ __global__ void __launch_bounds__(kDfThreads, 1) k_chol_dataflow(DevPlan d) {
       }
       __syncthreads();
       for (int u = 0; u < cnt; ++u) {
-        tile_sub_xyt<T>(A[t], W[2 * u], i == j ? W[2 * u] : W[2 * u + 1]);
+        if (i == j) tile_sub_sym(A[t], W[2 * u]); else tile_sub_xyt<T>(A[t], W[2 * u], W[2 * u + 1]);
         if (i == j && tid < kTile) {
           T tv = bown[t * kTile + tid];
 #pragma unroll 8
@@ -2445,81 +3141,24 @@ __global__ void __launch_bounds__(kDfThreads, 1) k_chol_dataflow(DevPlan d) {
       continue;
     }
     if (i == j) {                          // factor a diagonal tile
+      if (warp < 4 &&
+          !tile_potrf_inverse(A[t], Dinv, fb, Lg + (long long)i * kTile * kTile, warp, lane) && lane == 0)
+        s_ok = 0;
       if (!finish_diag(t, i)) break;
       ++ndone;
       __syncthreads();
       continue;
     }
-    // panel L_ij = A_ij L_jj^-T, kept in A[t] (kChain2: after the update
-    // from column j-1)
-    const bool chain = mode == kChain || mode == kChain2;
-    {
-      TileFetch<T> f, fi, fj;
-      const T* Li = Lg + (long long)j * kTile * kTile;
-#pragma unroll
-      for (int u = 0; u < kPerThread; ++u) f.v[u] = __ldcg(Li + threadIdx.x + u * kCholThreads);
-      if (mode == kChain2) {
-        fetch_rect_cg<T>(fi, S, n, i, j - 1);
-        fetch_rect_cg<T>(fj, S, n, j, j - 1);
-      }
-      T yj = T(0);
-      if (chain && tid < kTile) yj = __ldcg(b + kTile * j + tid);
-      f.store(Dinv);
-      if (mode == kChain2) {
-        fi.store(W[0]);
-        fj.store(W[1]);
-      }
-      if (chain && tid < kTile) yv[0][tid] = yj;
-    }
-    __syncthreads();
-    if (mode == kChain2) {
-      tile_sub_xyt<T>(A[t], W[0], W[1]);
-      __syncthreads();
-    }
-    {
-      T sv[8];
-      if (tid < 128) tile_xyt<T>(A[t], Dinv, sv);
-      __syncthreads();
-      if (tid < 128) {
-        const int r = tid >> 3, c0 = tid & 7;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          A[t][r][c0 + 8 * u] = sv[u];
-          A[t][r + 16][c0 + 8 * u] = sv[4 + u];
-        }
-      }
-    }
-    __syncthreads();
-    {
-      const int mi = tile_rows(n, i);
-      const int r = tid >> 3, c0 = tid & 7;
-      if (r < mi) {
-        T* row = S + (long long)(kTile * i + r) * n + kTile * j;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) row[c0 + 8 * u] = A[t][r][c0 + 8 * u];
-      }
-    }
-    if (chain) {
-      // the diagonal tile of row i: its last update (from this panel), then
-      // its factorization; both are announced together
-      const int td = pr_s[t];
-      tile_sub_xyt<T>(A[td], A[t], A[t]);
-      if (tid < kTile) {
-        T tv = bown[td * kTile + tid];
-#pragma unroll 8
-        for (int q = 0; q < kTile; ++q) tv -= A[t][tid][q] * yv[0][q];
-        bown[td * kTile + tid] = tv;
-      }
-      __syncthreads();
-      if (!finish_diag(td, i)) break;
+    if (mode == kChain) {
+      if (!chain_task(t, pr_s[t], i)) break;
       ++ndone;
     } else {
+      panel_of(A[t], j);
+      publish_panel(i, j, warp, 8);
       __syncthreads();
+      if (tid == 0) st_release_u32(flags + (long long)i * nt + j, epoch);
     }
-    if (tid == 0) {
-      st_release_u32(flags + (long long)i * nt + j, epoch);
-      kt_s[t] = j + 1;
-    }
+    if (tid == 0) kt_s[t] = j + 1;
     ++ndone;
     __syncthreads();
   }
@@ -2884,7 +3523,7 @@ __global__ void __launch_bounds__(kCholThreads, 1) k_chol_small(DevPlan d) {
   extern __shared__ __align__(16) unsigned char cs_raw[];
   __shared__ __align__(16) Tile<T> Dinv;
   __shared__ T bs[kSolveSmallTiles][kTile];   // b after the columns done so far
-  __shared__ T colbuf[4 * kTile + 8];
+  __shared__ PotrfBuf<T> fb;
   __shared__ int ok_s;
   Tile<T>* A = reinterpret_cast<Tile<T>*>(cs_raw);   // tile (i, j), j <= i, at i (i + 1) / 2 + j
   const int p = blockIdx.y;
@@ -2907,28 +3546,32 @@ __global__ void __launch_bounds__(kCholThreads, 1) k_chol_small(DevPlan d) {
       if (i == j) f.diag(S, n, i); else f.rect(S, n, i, j);
       f.store(at(i, j));
     }
+  if (tid == 0) {
+    ok_s = 1;
+    fb.step = 0;
+  }
   for (int e = tid; e < nt * kTile; e += blockDim.x) {
     const int t = e / kTile, r = e % kTile;
     bs[t][r] = r < tile_rows(n, t) ? b[kTile * t + r] : T(0);
   }
   __syncthreads();
   for (int c = 0; c < nt; ++c) {
-    if (warp < 2) {
-      const bool ok = pair_potrf_inverse<T>(at(c, c), Dinv, colbuf, colbuf + 4 * kTile, warp, lane);
-      if (warp == 0 && lane == 0) ok_s = ok ? 1 : 0;
+    if (warp < 4) {
+      if (!tile_potrf_inverse(at(c, c), Dinv, fb, Lg + (long long)c * kTile * kTile, warp, lane) && lane == 0)
+        ok_s = 0;
     }
     __syncthreads();
     if (!ok_s) {
       if (tid == 0) d.factor_flag[p] = 1;
       return;
     }
-    // L_cc^-1 out, y_c = L_cc^-1 b_c (b_c after the columns before c)
-    for (int e = tid; e < kTile * kTile; e += blockDim.x) Lg[(long long)c * kTile * kTile + e] = Dinv[e / kTile][e % kTile];
+    // y_c = L_cc^-1 b_c (b_c after the columns before c)
+    T* const ycol = &fb.f[0][0][0];   // (the factor's buffers are free again)
     if (tid < kTile) {
       T y = T(0);
 #pragma unroll 8
       for (int q = 0; q < kTile; ++q) y += Dinv[tid][q] * bs[c][q];
-      colbuf[tid] = y;   // (the factor's buffers are free again)
+      ycol[tid] = y;
     }
     // panels L_ic = A_ic L_cc^-T, two tiles at a time
     for (int i = c + 1 + (tid >> 7); i < nt; i += 2) {
@@ -2936,7 +3579,7 @@ __global__ void __launch_bounds__(kCholThreads, 1) k_chol_small(DevPlan d) {
       tile_xyt_t<T>(at(i, c), Dinv, sv, tid & 127);
       const int r = (tid & 127) >> 3, c0 = tid & 7;
       // every read of this tile precedes its writes within the thread group
-      asm volatile("bar.sync %0, 128;\n" ::"r"(2 + (tid >> 7)) : "memory");
+      asm volatile("bar.sync %0, 128;\n" ::"r"(kQuadBarrier + (tid >> 7)) : "memory");
 #pragma unroll
       for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -2944,8 +3587,8 @@ __global__ void __launch_bounds__(kCholThreads, 1) k_chol_small(DevPlan d) {
     }
     __syncthreads();
     if (tid < kTile) {
-      bs[c][tid] = colbuf[tid];
-      if (tid < tile_rows(n, c)) b[kTile * c + tid] = colbuf[tid];
+      bs[c][tid] = ycol[tid];
+      if (tid < tile_rows(n, c)) b[kTile * c + tid] = ycol[tid];
     }
     for (int i = c + 1; i < nt; ++i) {   // the panels into S for the backward solve
       const int mi = tile_rows(n, i);
@@ -3959,7 +4602,8 @@ int launch_cholesky_solve(const DevPlan& d, cudaStream_t s) {
 }
 
 template <typename T>
-bool dataflow_layout_t(int nt, int device, int* grid, int* max_own, std::vector<int>* own_off,
+bool dataflow_layout_t(int nt, int device, int* grid, int* max_own, int* rows, int* helpers,
+                       std::vector<int>* own_off,
                        std::vector<int2>* own) {
   int sms = 0, coop = 0, optin = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
@@ -3971,26 +4615,31 @@ bool dataflow_layout_t(int nt, int device, int* grid, int* max_own, std::vector<
   if (!coop || nt < 2) return false;
   const long long ntiles = (long long)nt * (nt + 1) / 2;
   const int G = int(std::min<long long>(sms, ntiles));
-  // row i's diagonal tile and its left neighbour go to CTA i mod G; the
-  // rest, heaviest first, to the CTA with the least work so far.  When
-  // there are at least twice as many CTAs as tile rows, the chain's CTAs
-  // take none of the rest: a CTA busy with an update when its row's chain
+  // row i's last tiles go to CTA i mod G; the rest, heaviest first, to the
+  // CTA with the least work so far.  When there are at least twice as many
+  // CTAs as tile rows, the rows' CTAs take none of the rest (and run the
+  // rows' fixed program): a CTA busy with an update when its row's chain
   // task becomes ready would delay the chain by that update
   std::vector<std::vector<int2>> lists(G);
-  const int first_worker = (G >= 2 * nt) ? nt : 0;
+  const bool dedicated = G >= 2 * nt;
+  const int row_tiles = dedicated ? df_row_tiles<T>() : 2;
+  const int helper_tiles = G >= 4 * nt ? df_helper_tiles<T>() : 0;
+  const int band = row_tiles + helper_tiles;   // tiles of a row kept by its own CTAs
+  *rows = dedicated ? nt : 0;
+  *helpers = helper_tiles > 0 ? nt : 0;
+  const int first_worker = *rows + *helpers;
   std::vector<long long> load(G, 0);
   for (int i = 0; i < nt; ++i) {
     const int g = i % G;
-    lists[g].push_back(make_int2(i, i));
-    load[g] += i + 1;
-    if (i > 0) {
-      lists[g].push_back(make_int2(i, i - 1));
-      load[g] += i;
+    for (int u = 0; u < row_tiles && u <= i; ++u) {
+      lists[g].push_back(make_int2(i, i - u));
+      load[g] += i - u + 1;
     }
+    for (int u = row_tiles; u < band && u <= i; ++u) lists[nt + i].push_back(make_int2(i, i - u));
   }
   std::vector<int2> rest;
   for (int j = 0; j < nt; ++j)
-    for (int i = j + 2; i < nt; ++i) rest.push_back(make_int2(i, j));
+    for (int i = j + band; i < nt; ++i) rest.push_back(make_int2(i, j));
   std::stable_sort(rest.begin(), rest.end(), [](const int2& a, const int2& b) { return a.y > b.y; });
   for (const int2& t : rest) {
     int g = first_worker;
@@ -4007,7 +4656,7 @@ bool dataflow_layout_t(int nt, int device, int* grid, int* max_own, std::vector<
     mo = std::max(mo, int(l.size()));
   }
   const size_t smem = df_smem_bytes<T>(mo);
-  if (smem > size_t(optin) || mo > kDfThreads) return false;
+  if (smem > size_t(optin) || mo > (dedicated ? 64 : kDfThreads)) return false;
   if (cudaFuncSetAttribute(reinterpret_cast<const void*>(&k_chol_dataflow<T>),
                            cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
     cudaGetLastError();
@@ -4030,10 +4679,10 @@ bool dataflow_layout_t(int nt, int device, int* grid, int* max_own, std::vector<
   return true;
 }
 
-bool dataflow_layout(int nt, bool mixed, int device, int* grid, int* max_own,
+bool dataflow_layout(int nt, bool mixed, int device, int* grid, int* max_own, int* rows, int* helpers,
                      std::vector<int>* own_off, std::vector<int2>* own) {
-  return mixed ? dataflow_layout_t<float>(nt, device, grid, max_own, own_off, own)
-               : dataflow_layout_t<double>(nt, device, grid, max_own, own_off, own);
+  return mixed ? dataflow_layout_t<float>(nt, device, grid, max_own, rows, helpers, own_off, own)
+               : dataflow_layout_t<double>(nt, device, grid, max_own, rows, helpers, own_off, own);
 }
 
 int launch_assemble_blocks(const DevPlan& d, cudaStream_t s) {

@@ -1574,12 +1574,14 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
     if (v >= 0) D.solve_drop_step = v;
   }
   if (!pcg && nprob == 1 && !opt.shared_device && max_nt >= 2) {
-    int grid = 0, mo = 0;
+    int grid = 0, mo = 0, rows = 0, helpers = 0;
     std::vector<int> own_off;
     std::vector<int2> own;
-    if (dataflow_layout(max_nt, mixed, device, &grid, &mo, &own_off, &own)) {
+    if (dataflow_layout(max_nt, mixed, device, &grid, &mo, &rows, &helpers, &own_off, &own)) {
       D.df_grid = grid;
       D.df_max_own = mo;
+      D.df_rows = rows;
+      D.df_helpers = helpers;
       // bounded waits: a CTA that finds nothing ready for this many polls
       // records GBA_ERR_TIMEOUT; GBA_DF_SPIN_LIMIT lowers it to test that path
       D.df_spin_limit = 1LL << 22;
