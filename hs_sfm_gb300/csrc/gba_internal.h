@@ -285,8 +285,8 @@ struct DevPlan {
   // fold_count [2B]: per problem the arrival counters of the two kernels.
   int fold_ctrl;
   unsigned* fold_count;
-  // batched dense factorization of small systems (at most 8 tile rows,
-  // FP32): one launch of k_chol_small (factor and solve) per iteration
+  // dense factorization of small systems (at most 8 tile rows, FP32,
+  // batched or alone): one launch of k_chol_small (factor and solve) per iteration
   // instead of the per-column launches
   int chol_small;
 };

@@ -2054,15 +2054,18 @@ __device__ __forceinline__ void tile_sub_sym(Tile<double>& A, const Tile<double>
 // (this one is the w-th): lane = row, warp w the columns 2 kWarps m + w and
 // 2 kWarps m + 2 kWarps - 1 - w (an even split of the triangle).  The terms
 // past a column's diagonal are zeros and are left out: the sums of tile_xyt
-// in half its products.  P may not be A.
+// in half its products.
+template <int kWarps>
+__device__ __forceinline__ int panel_col(int u, int w) { return kWarps * u + ((u & 1) ? kWarps - 1 - w : w); }
+
 template <typename T, int kWarps>
-__device__ __forceinline__ void tile_panel(const Tile<T>& A, const Tile<T>& Li, Tile<T>& P, int w, int lane) {
+__device__ __forceinline__ void tile_panel_sums(const Tile<T>& A, const Tile<T>& Li, int w, int lane,
+                                                T (&s)[kTile / kWarps]) {
   constexpr int N = Vec16<T>::N, C = kTile / kWarps;
   int col[C];
-  T s[C];
 #pragma unroll
   for (int u = 0; u < C; ++u) {
-    col[u] = kWarps * u + ((u & 1) ? kWarps - 1 - w : w);
+    col[u] = panel_col<kWarps>(u, w);
     s[u] = T(0);
   }
 #pragma unroll
@@ -2080,8 +2083,14 @@ __device__ __forceinline__ void tile_panel(const Tile<T>& A, const Tile<T>& Li, 
       }
     }
   }
+}
+// (P may not be A: other warps still read it)
+template <typename T, int kWarps>
+__device__ __forceinline__ void tile_panel(const Tile<T>& A, const Tile<T>& Li, Tile<T>& P, int w, int lane) {
+  T s[kTile / kWarps];
+  tile_panel_sums<T, kWarps>(A, Li, w, lane, s);
 #pragma unroll
-  for (int u = 0; u < C; ++u) P[lane][col[u]] = s[u];
+  for (int u = 0; u < kTile / kWarps; ++u) P[lane][panel_col<kWarps>(u, w)] = s[u];
 }
 
 // Factor the SPD tile D (lower triangle used; identity-padded) and write
@@ -2102,6 +2111,11 @@ __device__ __forceinline__ void bar_arrive(int id, int threads) {
   asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }
 
+// x > 0 without the FP64 pipe
+__device__ __forceinline__ bool positive64(double x) {
+  const long long b = __double_as_longlong(x);
+  return b > 0 && b <= 0x7ff0000000000000LL;
+}
 // (one evaluation for both: an FP64 instruction costs the same for one lane)
 __device__ __forceinline__ void rsqrt_two(double a, double b, double& ra, double& rb) {
   const double r = rsqrt((threadIdx.x & 1) ? b : a);
@@ -2120,7 +2134,6 @@ struct PotrfBuf<double> {
 template <>
 struct PotrfBuf<float> {
   alignas(16) float f[kTile / 2][2][kTile];   // the columns of L, pair by pair
-  float4 piv[kTile / 2];                        // r0, l10, r1 of each pair
   int step;                                     // pairs published so far
 };
 
@@ -2137,72 +2150,99 @@ __device__ __forceinline__ int ld_acquire_shared(const int* p) {
   return v;
 }
 
-// FP32: latency, not throughput, so one warp runs the whole chain of pivots
-// without ever waiting for another: lane i of warp 0 keeps row i of the tile
-// in registers, lane i of warp 1 column i of L^-1 (forward substitution
-// against L), one step behind.  A step's critical part goes through
-// shuffles only: the next pair's two columns are updated and its pivot block
-// read first, the rest of the trailing updates (from the published columns,
-// four to a load) fills the latency of the next pivots' square roots.  Warp
-// 1 waits for `step`, which warp 0 always reaches (it has no wait of its
-// own; the limit only makes the bound explicit).  16 pairs in 1.0 us; with the tile's columns spread over four
-// warps and a barrier a pair (the FP64 form) 2.2 us.
+// FP32: latency and one warp's issue slots.  Lane i of warp 0 keeps the
+// columns 0..15 of row i in registers, lane i of warp 2 the columns 16..31,
+// lane i of warp 1 column i of L^-1 (forward substitution against L).  Warp 0
+// runs the first eight pairs without ever waiting for another, warp 2 applies
+// each to its columns as it is published and then runs the last eight, warp 1
+// follows one step behind.  A step's critical part goes through shuffles:
+// the next pair's two columns are updated and its pivot block read first, the
+// half's other columns (from the published ones, four to a load) fill the
+// latency of the next square roots.  The waits (for `step`, which its owner
+// always reaches) are bounded all the same.  1,330 cycles; all 32 columns in
+// one warp took 2,630 (its issue slots), over four warps with a barrier a pair
+// (the FP64 form) 4,400.
+template <int B>
+__device__ __forceinline__ void potrf_half(float (&a)[kTile / 2], PotrfBuf<float>& fb, int lane, bool& ok) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int H = kTile / 2;
+  float p0 = __shfl_sync(FULL, a[0], B), p1 = __shfl_sync(FULL, a[0], B + 1), p2 = __shfl_sync(FULL, a[1], B + 1);
+  // every column index is a compile-time constant, so a[] stays in registers
+  static_for<0, H, 2>([&](auto hc) {
+    constexpr int h = decltype(hc)::value, j = B + h, s = j / 2;
+    const float det = fmaf(p0, p2, -(p1 * p1));
+    const float r0 = rsqrtf(p0), rd = rsqrtf(det);
+    const float l00 = p0 * r0;             // sqrt(p0)
+    const float l10 = p1 * r0;
+    const float r1 = l00 * rd;             // 1 / sqrt(det / p0)
+    ok = ok && (p0 > 0.0f) && (det > 0.0f);
+    const float li0 = lane > j ? a[h] * r0 : 0.0f;
+    const float li1 = lane > j + 1 ? fmaf(-li0, l10, a[h + 1]) * r1 : 0.0f;
+    // the diagonal's places carry the reciprocals for the inverse
+    fb.f[s][0][lane] = lane == j ? r0 : li0;
+    fb.f[s][1][lane] = lane == j + 1 ? r1 : li1;
+    if constexpr (h + 2 < H) {
+      const float c00 = __shfl_sync(FULL, li0, j + 2), c10 = __shfl_sync(FULL, li1, j + 2);
+      const float c01 = __shfl_sync(FULL, li0, j + 3), c11 = __shfl_sync(FULL, li1, j + 3);
+      a[h + 2] = fmaf(-li1, c10, fmaf(-li0, c00, a[h + 2]));
+      a[h + 3] = fmaf(-li1, c11, fmaf(-li0, c01, a[h + 3]));
+      p0 = __shfl_sync(FULL, a[h + 2], j + 2);
+      p1 = __shfl_sync(FULL, a[h + 2], j + 3);
+      p2 = __shfl_sync(FULL, a[h + 3], j + 3);
+    }
+    __syncwarp();
+    if (lane == 0) st_release_shared(&fb.step, s + 1);
+#pragma unroll
+    for (int l = (h + 4) / 4 * 4; l < H; l += 4) {
+      float c0[4], c1[4];
+      load16(&fb.f[s][0][B + l], c0);
+      load16(&fb.f[s][1][B + l], c1);
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (l + e >= h + 4) a[l + e] = fmaf(-li1, c1[e], fmaf(-li0, c0[e], a[l + e]));
+    }
+  });
+}
+
 __device__ __forceinline__ bool tile_potrf_inverse(const Tile<float>& D, Tile<float>& Dinv, PotrfBuf<float>& fb,
                                                    float* __restrict__ Lg, int warp, int lane) {
-  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int H = kTile / 2;
   bool ok = true;
-  if (warp == 0) {
-    float a[kTile];
+  auto wait_step = [&](int s) {
+    for (int spin = 0; ld_acquire_shared(&fb.step) <= s && ok; ++spin) ok = spin < (1 << 20);
+  };
+  if (warp == 0 || warp == 2) {
+    float a[H];
 #pragma unroll
-    for (int q = 0; q < kTile; q += 4) load16(&D[lane][q], a + q);
-    float p0 = __shfl_sync(FULL, a[0], 0), p1 = __shfl_sync(FULL, a[0], 1), p2 = __shfl_sync(FULL, a[1], 1);
-    // j is a compile-time constant in every step, so a[] stays in registers
-    static_for<0, kTile / 2, 1>([&](auto sc) {
-      constexpr int s = decltype(sc)::value, j = 2 * s;
-      const float det = fmaf(p0, p2, -(p1 * p1));
-      const float r0 = rsqrtf(p0), rd = rsqrtf(det);
-      const float l00 = p0 * r0;             // sqrt(p0)
-      const float l10 = p1 * r0;
-      const float r1 = l00 * rd;             // 1 / sqrt(det / p0)
-      ok = ok && (p0 > 0.0f) && (det > 0.0f);
-      // rows above the pair hold nothing here; the pair's own rows are not
-      // read by the trailing updates, which start below them
-      const float li0 = lane > j ? a[j] * r0 : 0.0f;
-      const float li1 = lane > j + 1 ? fmaf(-li0, l10, a[j + 1]) * r1 : 0.0f;
-      fb.f[s][0][lane] = li0;
-      fb.f[s][1][lane] = li1;
-      if (lane == 0) fb.piv[s] = make_float4(r0, l10, r1, 0.0f);
-      if constexpr (j + 2 < kTile) {
-        const float c00 = __shfl_sync(FULL, li0, j + 2), c10 = __shfl_sync(FULL, li1, j + 2);
-        const float c01 = __shfl_sync(FULL, li0, j + 3), c11 = __shfl_sync(FULL, li1, j + 3);
-        a[j + 2] = fmaf(-li1, c10, fmaf(-li0, c00, a[j + 2]));
-        a[j + 3] = fmaf(-li1, c11, fmaf(-li0, c01, a[j + 3]));
-        p0 = __shfl_sync(FULL, a[j + 2], j + 2);
-        p1 = __shfl_sync(FULL, a[j + 2], j + 3);
-        p2 = __shfl_sync(FULL, a[j + 3], j + 3);
-      }
-      __syncwarp();
-      if (lane == 0) st_release_shared(&fb.step, s + 1);
+    for (int q = 0; q < H; q += 4) load16(&D[lane][(warp == 0 ? 0 : H) + q], a + q);
+    if (warp == 0) {
+      potrf_half<0>(a, fb, lane, ok);
+    } else {
+      static_for<0, H / 2, 1>([&](auto sc) {
+        constexpr int s = decltype(sc)::value;
+        wait_step(s);
+        const float li0 = fb.f[s][0][lane], li1 = fb.f[s][1][lane];
 #pragma unroll
-      for (int l = (j + 4) / 4 * 4; l < kTile; l += 4) {
-        float c0[4], c1[4];
-        load16(&fb.f[s][0][l], c0);
-        load16(&fb.f[s][1][l], c1);
+        for (int l = 0; l < H; l += 4) {
+          float c0[4], c1[4];
+          load16(&fb.f[s][0][H + l], c0);
+          load16(&fb.f[s][1][H + l], c1);
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (l + e >= j + 4) a[l + e] = fmaf(-li1, c1[e], fmaf(-li0, c0[e], a[l + e]));
-      }
-    });
+          for (int e = 0; e < 4; ++e) a[l + e] = fmaf(-li1, c1[e], fmaf(-li0, c0[e], a[l + e]));
+        }
+      });
+      potrf_half<H>(a, fb, lane, ok);
+    }
   } else if (warp == 1) {
     float x[kTile];
 #pragma unroll
     for (int r = 0; r < kTile; ++r) x[r] = (r == lane) ? 1.0f : 0.0f;
     static_for<0, kTile / 2, 1>([&](auto sc) {
       constexpr int s = decltype(sc)::value, j = 2 * s;
-      for (int spin = 0; ld_acquire_shared(&fb.step) <= s && ok; ++spin) ok = spin < (1 << 20);
-      const float4 pv = fb.piv[s];   // r0, l10, r1
-      x[j] *= pv.x;
-      x[j + 1] = fmaf(-pv.y, x[j], x[j + 1]) * pv.z;
+      wait_step(s);
+      const float r0 = fb.f[s][0][j], l10 = fb.f[s][0][j + 1], r1 = fb.f[s][1][j + 1];
+      x[j] *= r0;
+      x[j + 1] = fmaf(-l10, x[j], x[j + 1]) * r1;
       Dinv[j][lane] = x[j];
       Dinv[j + 1][lane] = x[j + 1];
       if (Lg) {
@@ -2220,7 +2260,7 @@ __device__ __forceinline__ bool tile_potrf_inverse(const Tile<float>& D, Tile<fl
       }
     });
     __syncwarp();
-    if (lane == 0) fb.step = 0;   // warp 0 has published its last pair
+    if (lane == 0) fb.step = 0;   // every pair is published and warp 2 waits for none of them
   }
   return ok;
 }
@@ -2272,11 +2312,11 @@ __device__ __forceinline__ bool tile_potrf_inverse(const Tile<double>& D, Tile<d
       const T det = fma(p0, p2, -(p1 * p1));
       T r0, rd;
       rsqrt_two(p0, det, r0, rd);
-      const T l00 = p0 * r0;             // sqrt(p0)
-      const T l10 = p1 * r0;
-      const T r1 = l00 * rd;             // 1 / sqrt(det / p0)
-      ok = ok && (p0 > T(0)) && (det > T(0));
       const T f0 = lane == j ? r0 : a0 * r0;
+      const T l00 = p0 * r0;             // sqrt(p0)
+      const T l10 = __shfl_sync(FULL, f0, j + 1);   // p1 r0
+      const T r1 = l00 * rd;             // 1 / sqrt(det / p0)
+      ok = ok && positive64(p0) && positive64(det);
       const T f1 = lane == j + 1 ? r1 : fma(-f0, l10, a1) * r1;
       fb.f[s & 3][0][lane] = lane == j + 1 ? T(0) : f0;   // (row j of the inverse ends at j)
       fb.f[s & 3][1][lane] = f1;
@@ -3230,7 +3270,7 @@ __device__ __forceinline__ void chol_solve_body(const DevPlan& d, int q) {
   T cur[kTile];
   auto fetch = [&](int jj) {
     const int i = q + R * warp;
-    if (jj < 0 || i >= jj) return;
+    if (jj < 0 || i >= jj || warp >= 8) return;
     const int mj = tile_rows(n, jj);
     const T* row = S + (long long)kTile * jj * n + kTile * i + lane;
 #pragma unroll
@@ -3281,7 +3321,7 @@ __device__ __forceinline__ void chol_solve_body(const DevPlan& d, int q) {
       jown -= R;
       fetch_linv(jown);
     }
-    const int nact = j > q ? (j - q + R - 1) / R : 0;
+    const int nact = warp < 8 && j > q ? (j - q + R - 1) / R : 0;   // (eight warps; others only keep step)
     if (warp < nact) {
       T acc = T(0);
 #pragma unroll
@@ -3503,25 +3543,30 @@ __global__ void __launch_bounds__(256) k_chol_solve_small(DevPlan d) {
   chol_solve_body<T, 1>(d, 0);
 }
 
-// Batched factorization and solve of small reduced systems (at most
-// kSolveSmallTiles tile rows, FP32): one CTA per problem keeps the tiles of
-// the lower triangle in shared memory and runs the schedule of the
-// per-column launches (k_chol_step) inside the CTA -- for each column c the
-// diagonal tile's factor and inverse, the panels L_ic = A_ic L_cc^-T, the
-// forward-solve updates b_i -= L_ic y_c, then the trailing updates A_ij -=
-// L_ic L_jc^T, two tiles at a time -- with the same per-element arithmetic,
-// so the result has the bits of k_chol_step and k_chol_dataflow; then the
-// backward solve of k_chol_solve_small.  One launch per LM iteration
-// instead of one per tile column plus the solve.
+// Factorization and solve of small reduced systems (at most
+// kSolveSmallTiles tile rows, FP32), batched or alone: one CTA of 16 warps per
+// problem keeps the tiles of the lower triangle in shared memory and runs the
+// schedule of the per-column launches (k_chol_step) inside the CTA.  For each
+// column c: the panels L_ic = A_ic L_cc^-T, a tile to a group of four warps;
+// then group 0 updates the next diagonal tile and factors it while the other
+// groups take the rest of the trailing updates A_ij -= L_ic L_jc^T, the
+// panels into S and the forward-solve updates b_i -= L_ic y_c.  The
+// per-element arithmetic is that of k_chol_step, so the bits are those of
+// k_chol_step and k_chol_dataflow; then the backward solve of
+// k_chol_solve_small.  With two groups, one after the other through every
+// phase, 512 windows took 192 us an iteration.
+constexpr int kCholSmallThreads = 512;
+
 template <typename T>
 __host__ __device__ constexpr size_t chol_small_smem(int max_nt) {
   return size_t(max_nt) * (max_nt + 1) / 2 * sizeof(Tile<T>);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kCholThreads, 1) k_chol_small(DevPlan d) {
+__global__ void __launch_bounds__(kCholSmallThreads, 1) k_chol_small(DevPlan d) {
+  constexpr int kGroups = kCholSmallThreads / 128;
   extern __shared__ __align__(16) unsigned char cs_raw[];
-  __shared__ __align__(16) Tile<T> Dinv;
+  __shared__ __align__(16) Tile<T> Dinv[2];
   __shared__ T bs[kSolveSmallTiles][kTile];   // b after the columns done so far
   __shared__ PotrfBuf<T> fb;
   __shared__ int ok_s;
@@ -3538,14 +3583,39 @@ __global__ void __launch_bounds__(kCholThreads, 1) k_chol_small(DevPlan d) {
   T* S = tptr_mut<T>(d.S) + pi.s_off;
   T* b = tptr_mut<T>(d.b) + 6LL * pi.ext_begin;
   T* Lg = tptr_mut<T>(d.Linv) + (long long)p * d.max_nt * kTile * kTile;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = tid >> 7, gt = tid & 127, gw = warp & 3;
   auto at = [&](int i, int j) -> Tile<T>& { return A[i * (i + 1) / 2 + j]; };
-  for (int i = 0; i < nt; ++i)
-    for (int j = 0; j <= i; ++j) {
-      TileFetch<T> f;
-      if (i == j) f.diag(S, n, i); else f.rect(S, n, i, j);
-      f.store(at(i, j));
+  auto row_of = [](int lin) {   // the row of tile `lin` of a lower triangle
+    int i = 0;
+    while ((i + 1) * (i + 2) / 2 <= lin) ++i;
+    return i;
+  };
+  // the tiles, two per group in flight; a diagonal tile keeps its lower
+  // triangle and has identity rows past the matrix
+  const int ntiles = nt * (nt + 1) / 2;
+  for (int lin0 = g; lin0 < ntiles; lin0 += 2 * kGroups) {
+    T v[2][8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int lin = lin0 + h * kGroups;
+      if (lin >= ntiles) continue;
+      const int i = row_of(lin), j = lin - i * (i + 1) / 2, mi = tile_rows(n, i);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int r = gw + 4 * u;
+        const bool in = r < mi && (i != j || lane <= r);
+        v[h][u] = in ? S[(long long)(kTile * i + r) * n + kTile * j + lane]
+                     : (i == j && r >= mi && r == lane ? T(1) : T(0));
+      }
     }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int lin = lin0 + h * kGroups;
+      if (lin >= ntiles) continue;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) A[lin][gw + 4 * u][lane] = v[h][u];
+    }
+  }
   if (tid == 0) {
     ok_s = 1;
     fb.step = 0;
@@ -3555,66 +3625,67 @@ __global__ void __launch_bounds__(kCholThreads, 1) k_chol_small(DevPlan d) {
     bs[t][r] = r < tile_rows(n, t) ? b[kTile * t + r] : T(0);
   }
   __syncthreads();
-  for (int c = 0; c < nt; ++c) {
-    if (warp < 4) {
-      if (!tile_potrf_inverse(at(c, c), Dinv, fb, Lg + (long long)c * kTile * kTile, warp, lane) && lane == 0)
-        ok_s = 0;
+  auto factor = [&](int c) {   // group 0
+    if (!tile_potrf_inverse(at(c, c), Dinv[c & 1], fb, Lg + (long long)c * kTile * kTile, gw, lane) && lane == 0)
+      ok_s = 0;
+  };
+  for (int c = -1; c < nt; ++c) {
+    if (c >= 0) {
+      // panels, a tile to a group; y_c = L_cc^-1 b_c (b_c after the columns before c)
+      const Tile<T>& Li = Dinv[c & 1];
+      for (int i = c + 1 + g; i < nt; i += kGroups) {
+        T sv[kTile / 4];
+        tile_panel_sums<T, 4>(at(i, c), Li, gw, lane, sv);
+        bar_sync(kQuadBarrier + g, 128);   // every read of this tile precedes its writes
+#pragma unroll
+        for (int u = 0; u < kTile / 4; ++u) at(i, c)[lane][panel_col<4>(u, gw)] = sv[u];
+      }
+      if (warp == 15) {
+        T y = T(0);
+#pragma unroll 8
+        for (int q = 0; q < kTile; ++q) y += Li[lane][q] * bs[c][q];
+        __syncwarp();
+        bs[c][lane] = y;
+        if (lane < tile_rows(n, c)) b[kTile * c + lane] = y;
+      }
+      __syncthreads();
+    }
+    if (c + 1 < nt) {
+      if (g == 0) {
+        if (c >= 0) {
+          tile_sub_sym(at(c + 1, c + 1), at(c + 1, c));
+          bar_sync(kQuadBarrier, 128);
+        }
+        factor(c + 1);
+      } else if (c >= 0) {
+        // the other trailing tiles (lin 0 is the next diagonal one)
+        const int m = nt - c - 1, ntr = m * (m + 1) / 2;
+        for (int lin = g; lin < ntr; lin += kGroups - 1) {
+          const int ti = row_of(lin), i = c + 1 + ti, j = c + 1 + (lin - ti * (ti + 1) / 2);
+          tile_sub_xyt_t<T>(at(i, j), at(i, c), at(j, c), gt);
+        }
+        // the panels into S for the backward solve, b_i -= L_ic y_c below
+        for (int i = c + g; i < nt; i += kGroups - 1) {
+          const int mi = tile_rows(n, i);
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const int r = gw + 4 * u;
+            if (r < mi) S[(long long)(kTile * i + r) * n + kTile * c + lane] = at(i, c)[r][lane];
+          }
+          if (gw == 3) {
+            T t = bs[i][lane];
+#pragma unroll 8
+            for (int q = 0; q < kTile; ++q) t -= at(i, c)[lane][q] * bs[c][q];
+            bs[i][lane] = t;
+          }
+        }
+      }
     }
     __syncthreads();
     if (!ok_s) {
       if (tid == 0) d.factor_flag[p] = 1;
       return;
     }
-    // y_c = L_cc^-1 b_c (b_c after the columns before c)
-    T* const ycol = &fb.f[0][0][0];   // (the factor's buffers are free again)
-    if (tid < kTile) {
-      T y = T(0);
-#pragma unroll 8
-      for (int q = 0; q < kTile; ++q) y += Dinv[tid][q] * bs[c][q];
-      ycol[tid] = y;
-    }
-    // panels L_ic = A_ic L_cc^-T, two tiles at a time
-    for (int i = c + 1 + (tid >> 7); i < nt; i += 2) {
-      T sv[8];
-      tile_xyt_t<T>(at(i, c), Dinv, sv, tid & 127);
-      const int r = (tid & 127) >> 3, c0 = tid & 7;
-      // every read of this tile precedes its writes within the thread group
-      asm volatile("bar.sync %0, 128;\n" ::"r"(kQuadBarrier + (tid >> 7)) : "memory");
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) at(i, c)[r + 16 * h][c0 + 8 * u] = sv[4 * h + u];
-    }
-    __syncthreads();
-    if (tid < kTile) {
-      bs[c][tid] = ycol[tid];
-      if (tid < tile_rows(n, c)) b[kTile * c + tid] = ycol[tid];
-    }
-    for (int i = c + 1; i < nt; ++i) {   // the panels into S for the backward solve
-      const int mi = tile_rows(n, i);
-      for (int e = tid; e < kTile * kTile; e += blockDim.x) {
-        const int r = e / kTile, q = e % kTile;
-        if (r < mi) S[(long long)(kTile * i + r) * n + kTile * c + q] = at(i, c)[r][q];
-      }
-    }
-    __syncthreads();
-    // forward-solve updates of the rows below: b_i -= L_ic y_c
-    for (int e = tid; e < (nt - c - 1) * kTile; e += blockDim.x) {
-      const int i = c + 1 + e / kTile, r = e % kTile;
-      T t = bs[i][r];
-#pragma unroll 8
-      for (int q = 0; q < kTile; ++q) t -= at(i, c)[r][q] * bs[c][q];
-      bs[i][r] = t;
-    }
-    // trailing updates A_ij -= L_ic L_jc^T, c < j <= i, two tiles at a time
-    const int m = nt - c - 1, ntr = m * (m + 1) / 2;
-    for (int lin = tid >> 7; lin < ntr; lin += 2) {
-      int ti = 0;
-      while ((ti + 1) * (ti + 2) / 2 <= lin) ++ti;
-      const int i = c + 1 + ti, j = c + 1 + (lin - ti * (ti + 1) / 2);
-      tile_sub_xyt_t<T>(at(i, j), at(i, c), at(j, c), tid & 127);
-    }
-    __syncthreads();
   }
   chol_solve_body<T, 1>(d, 0);
 }
@@ -4368,7 +4439,7 @@ template <typename T>
 int run_cholesky_factor(const DevPlan& d, cudaStream_t s) {
   if (d.chol_small) {   // factor and solve in one launch (small systems, FP32)
     if constexpr (sizeof(T) == sizeof(float))
-      k_chol_small<T><<<dim3(1u, unsigned(d.B)), kCholThreads, chol_small_smem<T>(d.max_nt), s>>>(d);
+      k_chol_small<T><<<dim3(1u, unsigned(d.B)), kCholSmallThreads, chol_small_smem<T>(d.max_nt), s>>>(d);
     return 1;
   }
   if (d.df_grid > 0) {
@@ -4565,6 +4636,28 @@ int launch_cholesky_factor(const DevPlan& d, cudaStream_t s) {
   return n;
 }
 
+// Allows a kernel all the dynamic shared memory its static arrays leave of the
+// device's limit (the limit is the function's, shared by every plan, so it is
+// never set to one plan's need); false when `need` bytes do not fit.
+static bool allow_dynamic_smem(const void* fn, size_t need) {
+  cudaFuncAttributes a = {};
+  int dev = 0, optin = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaFuncGetAttributes(&a, fn) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const long long most = (long long)optin - (long long)a.sharedSizeBytes;
+  if ((long long)need > most) return false;
+  if (a.maxDynamicSharedSizeBytes < most &&
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return true;
+}
+
 int prepare_cholesky_solve(int max_nt, int precision) {
   if (max_nt <= kSolveSmallTiles) return GBA_OK;
   const bool mixed = precision == GBA_PRECISION_MIXED;
@@ -4575,23 +4668,13 @@ int prepare_cholesky_solve(int max_nt, int precision) {
                       mixed ? reinterpret_cast<const void*>(&k_chol_solve<float, true>)
                             : reinterpret_cast<const void*>(&k_chol_solve<double, true>)};
   for (const void* fn : f)
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) != cudaSuccess) {
-      cudaGetLastError();
-      return GBA_ERR_UNSUPPORTED;
-    }
+    if (!allow_dynamic_smem(fn, bytes)) return GBA_ERR_UNSUPPORTED;
   return GBA_OK;
 }
 
 bool prepare_chol_small(int max_nt, int precision) {
   if (precision != GBA_PRECISION_MIXED || max_nt < 1 || max_nt > kSolveSmallTiles) return false;
-  const size_t bytes = chol_small_smem<float>(max_nt);
-  if (bytes > 48 * 1024 &&
-      cudaFuncSetAttribute(&k_chol_small<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) !=
-          cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return true;
+  return allow_dynamic_smem(reinterpret_cast<const void*>(&k_chol_small<float>), chol_small_smem<float>(max_nt));
 }
 
 int launch_cholesky_solve(const DevPlan& d, cudaStream_t s) {
@@ -4605,10 +4688,9 @@ template <typename T>
 bool dataflow_layout_t(int nt, int device, int* grid, int* max_own, int* rows, int* helpers,
                        std::vector<int>* own_off,
                        std::vector<int2>* own) {
-  int sms = 0, coop = 0, optin = 0;
+  int sms = 0, coop = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess ||
-      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) {
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
@@ -4656,12 +4738,9 @@ bool dataflow_layout_t(int nt, int device, int* grid, int* max_own, int* rows, i
     mo = std::max(mo, int(l.size()));
   }
   const size_t smem = df_smem_bytes<T>(mo);
-  if (smem > size_t(optin) || mo > (dedicated ? 64 : kDfThreads)) return false;
-  if (cudaFuncSetAttribute(reinterpret_cast<const void*>(&k_chol_dataflow<T>),
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
-    cudaGetLastError();
+  if (mo > (dedicated ? 64 : kDfThreads) ||
+      !allow_dynamic_smem(reinterpret_cast<const void*>(&k_chol_dataflow<T>), smem))
     return false;
-  }
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_chol_dataflow<T>, kDfThreads, smem) !=
           cudaSuccess || per_sm < 1) {

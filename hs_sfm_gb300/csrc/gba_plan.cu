@@ -1573,7 +1573,15 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
     const int v = std::atoi(ds);
     if (v >= 0) D.solve_drop_step = v;
   }
-  if (!pcg && nprob == 1 && !opt.shared_device && max_nt >= 2) {
+  // Small FP32 systems: one factor-and-solve launch, a CTA per problem
+  // (GBA_CHOL_COLUMNS=1 keeps the per-column launches, for comparison).  A
+  // system alone on the device takes it up to four tile rows (21 images: 27 us
+  // against 34 for the dataflow launch and the solve; at five 35 against 39,
+  // but its iteration is no faster, at eight 77 against 54).
+  const bool dataflow = !pcg && nprob == 1 && !opt.shared_device && max_nt >= 2;
+  D.chol_small = !pcg && !(dataflow && max_nt > 4) && std::getenv("GBA_CHOL_COLUMNS") == nullptr &&
+                 prepare_chol_small(max_nt, opt.precision);
+  if (dataflow && !D.chol_small) {
     int grid = 0, mo = 0, rows = 0, helpers = 0;
     std::vector<int> own_off;
     std::vector<int2> own;
@@ -1602,10 +1610,6 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
       }
     }
   }
-  // batched small systems: one factor-and-solve launch (GBA_CHOL_COLUMNS=1
-  // keeps the per-column launches, for comparison)
-  D.chol_small = !pcg && D.df_grid == 0 && std::getenv("GBA_CHOL_COLUMNS") == nullptr &&
-                 prepare_chol_small(max_nt, opt.precision);
   D.blk_map = dev_blocks && !pcg ? dv_bid : arena.upload(blk_map);
   int dev_pair_bad = 0;
   int* d_pair_bad = nullptr;
