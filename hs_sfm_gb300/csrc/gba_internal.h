@@ -74,7 +74,7 @@ struct LMState {
   int factor_ok;  // reduced system factored this iteration
   int first;      // the first linearization (sets mu0)
   int pcg_iters;
-  int pad_;
+  int loop_passes;  // problem 0: passes of the run's device-side iteration loop
 };
 
 // Per-problem constant description (device).
@@ -306,7 +306,9 @@ int launch_ctrl_initial_cost(const DevPlan& d, cudaStream_t s);
 // accepted candidate's cost)
 int launch_linearize(const DevPlan& d, cudaStream_t s, bool keys = true);
 int launch_image_reduce(const DevPlan& d, cudaStream_t s);
-int launch_ctrl_after_linearize(const DevPlan& d, cudaStream_t s);
+// loop (or null): the while node whose body this launch is in; it is told
+// whether any problem still iterates
+int launch_ctrl_after_linearize(const DevPlan& d, cudaStream_t s, const cudaGraphConditionalHandle* loop = nullptr);
 int launch_point_schur(const DevPlan& d, cudaStream_t s);
 // plan build with Z planes: key_slot [K] = the inverse of img_keys, and the
 // assembly's pairs rewritten as slots
@@ -317,7 +319,8 @@ int launch_assemble_S(const DevPlan& d, cudaStream_t s);
 int launch_cholesky(const DevPlan& d, cudaStream_t s);
 int launch_assemble_blocks(const DevPlan& d, cudaStream_t s);
 int launch_pcg_setup(const DevPlan& d, cudaStream_t s);
-int launch_pcg_iterations(const DevPlan& d, cudaStream_t s);
+// nested: inside the body of the iteration loop
+int launch_pcg_iterations(const DevPlan& d, cudaStream_t s, bool nested = false);
 int launch_cholesky_factor(const DevPlan& d, cudaStream_t s);
 int launch_cholesky_solve(const DevPlan& d, cudaStream_t s);
 // Raises the backward solve's shared-memory limit for systems of up to

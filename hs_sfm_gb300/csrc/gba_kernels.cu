@@ -4011,6 +4011,10 @@ __global__ void __launch_bounds__(32) k_pcg_loop_ctrl(DevPlan d, cudaGraphCondit
   }
 }
 
+// A loop inside another loop's body: a node's condition takes its default
+// only when the whole graph is launched, so it is opened before each solve.
+__global__ void k_pcg_loop_open(cudaGraphConditionalHandle h) { cudaGraphSetConditional(h, 1u); }
+
 // ---------------------------------------------------------------------------
 // back-substitution and update
 // ---------------------------------------------------------------------------
@@ -4224,9 +4228,8 @@ __global__ void __launch_bounds__(kCtrlThreads) k_ctrl_initial_cost(DevPlan d) {
   }
 }
 
-__global__ void k_ctrl_after_linearize(DevPlan d) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= d.B) return;
+// The checks after problem p's linearization; whether it goes on.
+__device__ __forceinline__ bool ctrl_after_linearize(const DevPlan& d, int p) {
   LMState& st = d.state[p];
   if (st.relin && st.active) {
     const double ginf = bitsd(st.ginf_bits);
@@ -4243,6 +4246,27 @@ __global__ void k_ctrl_after_linearize(DevPlan d) {
   if (st.active && st.iter >= d.max_iterations) {
     st.active = 0;
     st.stop = GBA_STOP_MAX_ITERATIONS;
+  }
+  return st.active != 0;
+}
+
+__global__ void k_ctrl_after_linearize(DevPlan d) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < d.B) ctrl_after_linearize(d, p);
+}
+
+// The same in one CTA, inside the body of the iteration loop (a CUDA-graph
+// while node): the loop goes on while any problem does.  The pass in which the
+// last problem stops finds nothing to do in its other stages.  (Every pass of
+// an active problem counts an iteration; the bound on the passes only makes
+// the loop's end explicit.)
+__global__ void __launch_bounds__(256) k_ctrl_loop(DevPlan d, cudaGraphConditionalHandle h) {
+  int any = 0;
+  for (int p = threadIdx.x; p < d.B; p += blockDim.x) any |= ctrl_after_linearize(d, p);
+  any = __syncthreads_or(any);
+  if (threadIdx.x == 0) {
+    const int passes = ++d.state[0].loop_passes;
+    cudaGraphSetConditional(h, any && passes <= d.max_iterations ? 1u : 0u);
   }
 }
 
@@ -4569,7 +4593,11 @@ int launch_image_reduce(const DevPlan& d, cudaStream_t s) {
   return 5;
 }
 
-int launch_ctrl_after_linearize(const DevPlan& d, cudaStream_t s) {
+int launch_ctrl_after_linearize(const DevPlan& d, cudaStream_t s, const cudaGraphConditionalHandle* loop) {
+  if (loop) {
+    k_ctrl_loop<<<1, 256, 0, s>>>(d, *loop);
+    return 1;
+  }
   k_ctrl_after_linearize<<<(d.B + 127) / 128, 128, 0, s>>>(d);
   return 1;
 }
@@ -4778,7 +4806,7 @@ int launch_pcg_setup(const DevPlan& d, cudaStream_t s) {
   return 2;
 }
 
-int launch_pcg_iterations(const DevPlan& d, cudaStream_t s) {
+int launch_pcg_iterations(const DevPlan& d, cudaStream_t s, bool nested) {
   if (d.I_ext <= 0) return 0;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (d.pcg_it && d.pcg_body_stream && cudaStreamIsCapturing(s, &cs) == cudaSuccess &&
@@ -4794,6 +4822,11 @@ int launch_pcg_iterations(const DevPlan& d, cudaStream_t s) {
     if (cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, nullptr, &nd) != cudaSuccess ||
         cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault) != cudaSuccess)
       throw CudaError{GBA_ERR_CUDA};
+    if (nested) {
+      k_pcg_loop_open<<<1, 1, 0, s>>>(h);
+      if (cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, nullptr, &nd) != cudaSuccess)
+        throw CudaError{GBA_ERR_CUDA};
+    }
     cp.type = cudaGraphNodeTypeConditional;
     cp.conditional.handle = h;
     cp.conditional.type = cudaGraphCondTypeWhile;
@@ -4812,7 +4845,7 @@ int launch_pcg_iterations(const DevPlan& d, cudaStream_t s) {
     if (cudaStreamEndCapture(bs, &body) != cudaSuccess ||
         cudaStreamUpdateCaptureDependencies(s, &node, nullptr, 1, cudaStreamSetCaptureDependencies) != cudaSuccess)
       throw CudaError{GBA_ERR_CUDA};
-    return 5;   // (one pass of the body; it runs as many passes as the solve needs)
+    return nested ? 6 : 5;   // (one pass of the body; it runs as many passes as the solve needs)
   }
   for (int it = 0; it < d.pcg_max_iterations; ++it) {
     GBA_DISPATCH(d, (k_pcg_spmv<T><<<d.n_ext_chunks, 256, 0, s>>>(d, it, 0)));

@@ -391,6 +391,10 @@ struct Plan {
   cudaStream_t side_stream = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   unsigned long long pcg_extra_seen = 0;
+  // the device-side iteration loop: the stream its body is captured on, and
+  // whether the last run's passes beyond the first are still to be counted
+  cudaStream_t loop_stream = nullptr;
+  bool passes_pending = false;
   bool ran = false;
   long long launches_last_run = 0;
   double setup_ms = 0;
@@ -437,6 +441,7 @@ struct Plan {
     arena.release();
     if (stream) cudaStreamDestroy(stream);
     if (pcg_stream) cudaStreamDestroy(pcg_stream);
+    if (loop_stream) cudaStreamDestroy(loop_stream);
     if (side_stream) cudaStreamDestroy(side_stream);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
@@ -451,7 +456,11 @@ struct Plan {
   // control (beside the point Schur and the assembly, which do not need
   // them); kEpilogue runs them for the last iteration
   enum Part { kAll, kPrologue, kIteration, kEpilogue };
-  void enqueue(bool profile, Part part = kAll);
+  void enqueue(bool profile, Part part = kAll, cudaStream_t on = nullptr,
+               const cudaGraphConditionalHandle* loop = nullptr);
+  bool iterates_in_loop() const;
+  void capture_loop();
+  void count_passes(int passes);
   int run();
   int sync();
 };
@@ -1770,10 +1779,63 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
   return GBA_OK;
 }
 
+// Whether a run's iterations are a device-side loop: when a stopping test
+// may end them early.  Unrolled, the launches after the last problem's stop
+// find nothing to do but still take about 2 us each (a small FP64 problem of
+// 8 iterations spent 1.3 ms of 2.8 in the other 42 of its 50).  A fixed number
+// of iterations keeps the unrolled sequence, whose launches follow each other
+// without the loop's turns.  GBA_UNROLLED=1 keeps it always, for comparison.
+bool Plan::iterates_in_loop() const {
+  return !opt.profile && opt.max_iterations >= 4 &&
+         (opt.eps1 > 0.0 || opt.eps2 > 0.0 || opt.function_tolerance > 0.0) &&
+         std::getenv("GBA_UNROLLED") == nullptr;
+}
+
+// Adds the iteration loop to the graph `stream` is being captured into: a
+// while node whose body is one iteration (with the previous linearization's
+// sums and checks first, which also serve as the epilogue).
+void Plan::capture_loop() {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaGraph_t g = nullptr;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t nd = 0;
+  GBA_CUDA(cudaStreamGetCaptureInfo(stream, &cs, nullptr, &g, &deps, nullptr, &nd));
+  cudaGraphConditionalHandle h = 0;
+  GBA_CUDA(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
+  cudaGraphNodeParams cp = {};
+  cp.type = cudaGraphNodeTypeConditional;
+  cp.conditional.handle = h;
+  cp.conditional.type = cudaGraphCondTypeWhile;
+  cp.conditional.size = 1;
+  cudaGraphNode_t node = nullptr;
+  GBA_CUDA(cudaGraphAddNode(&node, g, deps, nullptr, nd, &cp));
+  if (!loop_stream) GBA_CUDA(cudaStreamCreateWithFlags(&loop_stream, cudaStreamNonBlocking));
+  GBA_CUDA(cudaStreamBeginCaptureToGraph(loop_stream, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                         cudaStreamCaptureModeThreadLocal));
+  cudaGraph_t body = nullptr;
+  try {
+    enqueue(false, kIteration, loop_stream, &h);
+  } catch (...) {
+    cudaStreamEndCapture(loop_stream, &body);
+    throw;
+  }
+  GBA_CUDA(cudaStreamEndCapture(loop_stream, &body));
+  GBA_CUDA(cudaStreamUpdateCaptureDependencies(stream, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
+}
+
+// The loop ran `passes` passes in the last run; one is counted already.
+void Plan::count_passes(int passes) {
+  if (!passes_pending) return;
+  passes_pending = false;
+  const long long extra = iter_launches * (long long)(passes - 1);
+  launches_last_run += extra;
+  g_launches += extra;
+}
+
 // The launch sequence of one solve.  When profiling, an event is recorded
 // after each stage and tagged with it.
-void Plan::enqueue(bool profile, Part part) {
-  cudaStream_t s = stream;
+void Plan::enqueue(bool profile, Part part, cudaStream_t on, const cudaGraphConditionalHandle* loop) {
+  cudaStream_t s = on ? on : stream;
   long long n = 0;
   const bool prologue = part == kAll || part == kPrologue;
   const int iterations = part == kAll ? opt.max_iterations : (part == kIteration ? 1 : 0);
@@ -1818,12 +1880,12 @@ void Plan::enqueue(bool profile, Part part) {
       GBA_CUDA(cudaEventRecord(ev_fork, s));
       GBA_CUDA(cudaStreamWaitEvent(side_stream, ev_fork, 0));
       n += launch_image_reduce(d, side_stream);
-      n += launch_ctrl_after_linearize(d, side_stream);
+      n += launch_ctrl_after_linearize(d, side_stream, loop);
       GBA_CUDA(cudaEventRecord(ev_join, side_stream));
     } else {
       n += launch_image_reduce(d, s);
       mark(GBA_STAGE_IMAGE_REDUCE);
-      n += launch_ctrl_after_linearize(d, s);
+      n += launch_ctrl_after_linearize(d, s, loop);
       mark(GBA_STAGE_CONTROL);
     }
     n += launch_point_schur(d, s);
@@ -1836,7 +1898,7 @@ void Plan::enqueue(bool profile, Part part) {
       mark(GBA_STAGE_OTHER);
       n += launch_pcg_setup(d, s);
       mark(GBA_STAGE_FACTOR);
-      n += launch_pcg_iterations(d, s);
+      n += launch_pcg_iterations(d, s, loop != nullptr);
       mark(GBA_STAGE_SOLVE);
     } else {
       n += launch_assemble_S(d, s);
@@ -1885,12 +1947,22 @@ int Plan::run() {
   GBA_CUDA(cudaSetDevice(device));
   cudaGetLastError();   // a stale error from other code on this thread is not ours
   GBA_CUDA(cudaEventRecord(ev0, stream));
+  const bool loop = iterates_in_loop();
+  passes_pending = loop;
   if (opt.use_cuda_graph) {
     if (!graph_exec) {
       cudaGraph_t g;
       GBA_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
       try {
-        enqueue(profile);
+        if (loop) {
+          enqueue(false, kPrologue);
+          const long long pro = launches_last_run;
+          capture_loop();
+          iter_launches = launches_last_run;
+          launches_last_run += pro;
+        } else {
+          enqueue(profile);
+        }
       } catch (...) {
         cudaStreamEndCapture(stream, &g);
         throw;
@@ -1905,14 +1977,17 @@ int Plan::run() {
   } else if (!profile && opt.max_iterations > 0) {
     // one-shot: the prologue launched directly, then one LM iteration
     // captured once (its launches do not depend on the iteration) and
-    // replayed max_iterations times
+    // replayed max_iterations times, or in a loop
     enqueue(false, kPrologue);
     const long long pro = launches_last_run;
     if (!iter_exec) {
       cudaGraph_t g;
       GBA_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
       try {
-        enqueue(false, kIteration);
+        if (loop)
+          capture_loop();
+        else
+          enqueue(false, kIteration);
       } catch (...) {
         cudaStreamEndCapture(stream, &g);
         throw;
@@ -1922,9 +1997,14 @@ int Plan::run() {
       cudaGraphDestroy(g);
       iter_launches = launches_last_run;
     }
-    for (int it = 0; it < opt.max_iterations; ++it) GBA_CUDA(cudaGraphLaunch(iter_exec, stream));
-    enqueue(false, kEpilogue);
-    launches_last_run += pro + iter_launches * opt.max_iterations;
+    if (loop) {
+      GBA_CUDA(cudaGraphLaunch(iter_exec, stream));
+      launches_last_run = pro + iter_launches;
+    } else {
+      for (int it = 0; it < opt.max_iterations; ++it) GBA_CUDA(cudaGraphLaunch(iter_exec, stream));
+      enqueue(false, kEpilogue);
+      launches_last_run += pro + iter_launches * opt.max_iterations;
+    }
   } else {
     enqueue(profile);
   }
@@ -1949,6 +2029,11 @@ int Plan::sync() {
     pcg_extra_seen = *h_pcg_extra;
     launches_last_run += extra;
     g_launches += extra;
+  }
+  if (passes_pending) {
+    LMState st;
+    GBA_CUDA(cudaMemcpy(&st, d.state, sizeof(st), cudaMemcpyDeviceToHost));
+    count_passes(st.loop_passes);
   }
   if (d.df_trace && !trace_path.empty()) write_trace();
   if (opt.profile) {
@@ -2246,6 +2331,7 @@ int get_all(gba::Plan& P, double* const* xs, gba_report* reports) {
     GBA_CUDA(cudaStreamSynchronize(P.stream));
     std::vector<gba::LMState> st(P.B);
     GBA_CUDA(cudaMemcpy(st.data(), P.d.state, sizeof(gba::LMState) * P.B, cudaMemcpyDeviceToHost));
+    P.count_passes(st[0].loop_passes);
     const long long np = 3LL * P.d.P, ni = 6LL * P.d.I, nc = P.d.free_cams ? 10LL * P.d.Ctot : 0;
     const size_t nx = size_t(np + ni + nc);
     gba::HostBuf<double> stage(nx);
@@ -2354,8 +2440,13 @@ int gba_plan_kernel_stats(gba_plan* p, int32_t stage, double* total_ms, int32_t*
 
 int gba_plan_last_run_launches(gba_plan* p, int64_t* n) {
   if (!p || !n) return GBA_ERR_INVALID;
-  *n = p->impl.launches_last_run;
-  return GBA_OK;
+  return guarded([&] {
+    // the loop's passes are known once the run is over
+    if (p->impl.passes_pending && gba_plan_query(p) == GBA_OK)
+      if (int e = p->impl.sync()) return e;
+    *n = p->impl.launches_last_run;
+    return GBA_OK;
+  });
 }
 
 int gba_plan_device_bytes(gba_plan* p, int64_t* bytes) {
@@ -2450,7 +2541,8 @@ int gba_solve_batch_into(const gba_problem* problems, const double* const* near_
   phase("x0 uploaded");
   if (!err) err = gba_plan_run(plan);
   phase("launched");
-  if (!err) err = gba_plan_synchronize(plan);
+  if (!err && (!plan->impl.passes_pending || plan->impl.h_pcg_extra))
+    err = gba_plan_synchronize(plan);   // (else get_all waits and counts the loop's passes)
   phase("solved");
   if (!err) err = get_all(plan->impl, x_out, reports);
   phase("x read back");
