@@ -203,6 +203,66 @@ __device__ double block_sum(double v, double* smem) {
   return r;
 }
 
+// The sums of N doubles per thread over the CTA (4 or 8 warps): thread e < N
+// returns the sum of value e (0 elsewhere), formed by the trees of block_sum.
+// One barrier and N + 3 (N > 1) FP64 additions a warp instead of 2 N barriers
+// and 5 N: the FP64 pipe takes 19 cycles of the SM for each, which was a third
+// of the back-substitution and a fifth of the mixed cost kernel on 512 windows.
+// smem [N * warps].
+template <int N>
+__device__ double block_sums(double (&v)[N], double* smem) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  int base, count;
+  warp_scatter_sums<N>(v, lane, base, count);
+#pragma unroll
+  for (int e = 0; e < warp_scatter_max(N); ++e)
+    if (e < count) smem[(base + e) * nw + w] = v[e];
+  __syncthreads();
+  if (threadIdx.x >= N) return 0.0;
+  const double* p = smem + threadIdx.x * nw;
+  return nw == 8 ? ((p[0] + p[4]) + (p[2] + p[6])) + ((p[1] + p[5]) + (p[3] + p[7]))
+                 : (p[0] + p[2]) + (p[1] + p[3]);
+}
+
+// Maxima over the CTA without the FP64 pipe: non-negative numbers are ordered
+// as their bits; negative ones and NaN count as 0 (as fmax from 0 does).
+__device__ __forceinline__ unsigned long long max_bits(float v) {
+  return __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(v, 0.0f)));
+}
+__device__ __forceinline__ unsigned long long max_bits(double v) {
+  const long long b = __double_as_longlong(v);
+  unsigned long long m = b > 0 && b <= 0x7ff0000000000000LL ? (unsigned long long)b : 0ull;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long q = __shfl_xor_sync(0xffffffffu, m, o);
+    m = q > m ? q : m;
+  }
+  return m;
+}
+__device__ __forceinline__ double max_value(unsigned long long bits, float) {
+  return double(__uint_as_float(unsigned(bits)));
+}
+__device__ __forceinline__ double max_value(unsigned long long bits, double) { return bitsd(bits); }
+// a and b over the CTA into *ma and *mb (as ordered bits, atomically), smem [2 * warps]
+template <typename T>
+__device__ void block_max2(T a, T b, unsigned long long* smem, unsigned long long* ma, unsigned long long* mb) {
+  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const unsigned long long wa = max_bits(a), wb = max_bits(b);
+  if ((threadIdx.x & 31) == 0) {
+    smem[w] = wa;
+    smem[nw + w] = wb;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    unsigned long long m = 0ull;
+    for (int i = 0; i < nw; ++i) {
+      const unsigned long long q = smem[threadIdx.x * nw + i];
+      m = q > m ? q : m;
+    }
+    atomicMax(threadIdx.x == 0 ? ma : mb, dbits(max_value(m, T(0))));
+  }
+}
+
 // Arrival of this CTA at problem p's counter after thread 0 has written the
 // CTA's partial sums; true in every thread of the CTA that arrives last of
 // `total` (which then runs the problem's LM control step and resets the
@@ -228,21 +288,6 @@ template <bool CG>
 __device__ void ctrl_step_body(const DevPlan& d, int p, double* red);
 template <bool CG>
 __device__ void ctrl_accept_body(const DevPlan& d, int p, double* red);
-
-__device__ double block_max(double v, double* smem) {
-  v = warp_max(v);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) smem[w] = v;
-  __syncthreads();
-  double r = 0;
-  if (w == 0) {
-    int nw = blockDim.x >> 5;
-    r = (l < nw) ? smem[l] : 0.0;
-    r = warp_max(r);
-  }
-  __syncthreads();
-  return r;
-}
 
 // Huber rho and IRLS weight of a squared whitened residual s (Ceres'
 // HuberLoss semantics, restated from camera_shared_ceres_optimizor.hpp:253).
@@ -971,12 +1016,9 @@ __global__ void __launch_bounds__(256) k_cost(DevPlan d, int which) {
       store_vec<4>(rw + 4LL * k, out);
     }
   }
-  const double tot = block_sum(acc, red);
-  const double tot_raw = block_sum(acc_raw, red);
-  if (threadIdx.x == 0) {
-    d.key_chunk_sum[2LL * blockIdx.x] = tot;
-    d.key_chunk_sum[2LL * blockIdx.x + 1] = tot_raw;
-  }
+  double sums[2] = {acc, acc_raw};
+  const double tot = block_sums<2>(sums, red);
+  if (threadIdx.x < 2) d.key_chunk_sum[2LL * blockIdx.x + threadIdx.x] = tot;
   if (which == 1 && d.fold_ctrl) {   // the accept decision in the last CTA of the problem
     __shared__ int last;
     const int p = ch.prob;
@@ -1067,12 +1109,9 @@ __global__ void __launch_bounds__(256) k_cost_ff(DevPlan d, int which) {
   // over the chunk (each thread its own keys and the residuals it just
   // wrote), so the cost loop keeps its register count
   if (which == 1 && d.fuse_lin) linearize_chunk<float>(d, ch, par);
-  const double tot = block_sum(double(acc.hi) + double(acc.lo), red);
-  const double tot_raw = block_sum(acc_raw, red);
-  if (threadIdx.x == 0) {
-    d.key_chunk_sum[2LL * blockIdx.x] = tot;
-    d.key_chunk_sum[2LL * blockIdx.x + 1] = tot_raw;
-  }
+  double sums[2] = {double(acc.hi) + double(acc.lo), acc_raw};
+  const double tot = block_sums<2>(sums, red);
+  if (threadIdx.x < 2) d.key_chunk_sum[2LL * blockIdx.x + threadIdx.x] = tot;
   if (which == 1 && d.fold_ctrl) {   // the accept decision in the last CTA of the problem
     __shared__ int last;
     const int p = ch.prob;
@@ -1085,12 +1124,12 @@ __global__ void __launch_bounds__(256) k_cost_ff(DevPlan d, int which) {
 // Per point: V_p = sum J_p^T J_p, g_p = sum J_p^T r from its keys' records.
 template <typename T>
 __global__ void __launch_bounds__(kPointChunk) k_point_reduce(DevPlan d) {
-  __shared__ double red[32];
+  __shared__ unsigned long long red[2 * kPointChunk / 32];
   const Chunk ch = d.pt_chunks[blockIdx.x];
   const LMState& st = d.state[ch.prob];
   if (!st.relin || !st.active) return;
   const int pt = ch.begin + threadIdx.x;
-  double vmax = 0.0, gmax = 0.0;
+  T vmax = T(0), gmax = T(0);
   if (pt < ch.end) {
     const T* __restrict__ JR = tptr<T>(d.JR[st.parity]);
     T V[6] = {0, 0, 0, 0, 0, 0}, g[3] = {0, 0, 0};
@@ -1140,16 +1179,11 @@ __global__ void __launch_bounds__(kPointChunk) k_point_reduce(DevPlan d) {
     }
     T pv[12] = {V[0], V[1], V[2], V[3], V[4], V[5], g[0], g[1], g[2], T(0), T(0), T(0)};
     store_vec<12>(tptr_mut<T>(d.PV) + 12LL * pt, pv);
-    vmax = fmax(fmax(double(V[0]), double(V[3])), double(V[5]));
-    gmax = fmax(fmax(fabs(double(g[0])), fabs(double(g[1]))), fabs(double(g[2])));
+    vmax = fmax(fmax(V[0], V[3]), V[5]);
+    gmax = fmax(fmax(fabs(g[0]), fabs(g[1])), fabs(g[2]));
   }
-  const double bv = block_max(vmax, red);
-  const double bg = block_max(gmax, red);
-  if (threadIdx.x == 0) {
-    LMState* sp = d.state + ch.prob;
-    atomicMax(&sp->maxdiag_bits, dbits(bv));
-    atomicMax(&sp->ginf_bits, dbits(bg));
-  }
+  LMState* sp = d.state + ch.prob;
+  block_max2(vmax, gmax, red, &sp->maxdiag_bits, &sp->ginf_bits);
 }
 
 // image reduce: U_i = sum J_i^T J_i, g_i = sum J_i^T r.  Each image's keys
@@ -4099,12 +4133,9 @@ __global__ void __launch_bounds__(kPointChunk) k_backsub(DevPlan d) {
         gd += double(pv[6 + a]) * dp[a];
       }
     }
-    double s0 = block_sum(dn2, red), s1 = block_sum(xn2, red), s2 = block_sum(gd, red);
-    if (threadIdx.x == 0) {
-      d.pt_chunk_sum[3LL * blockIdx.x] = s0;
-      d.pt_chunk_sum[3LL * blockIdx.x + 1] = s1;
-      d.pt_chunk_sum[3LL * blockIdx.x + 2] = s2;
-    }
+    double sums[3] = {dn2, xn2, gd};
+    const double tot = block_sums<3>(sums, red);
+    if (threadIdx.x < 3) d.pt_chunk_sum[3LL * blockIdx.x + threadIdx.x] = tot;
   } else {
     const int c = blockIdx.x - d.n_pt_chunks;
     const Chunk ch = d.img_chunks[c];
@@ -4122,14 +4153,11 @@ __global__ void __launch_bounds__(kPointChunk) k_backsub(DevPlan d) {
       if (free_img) xn2 += xv * xv;
       gd += d.gi[e] * dv;
     }
-    double s0 = block_sum(dn2, red), s1 = block_sum(xn2, red), s2 = block_sum(gd, red);
-    // the candidate's rotations (block_sum's barriers made x_img[1 - par] visible)
+    double sums[3] = {dn2, xn2, gd};
+    const double tot = block_sums<3>(sums, red);
+    // the candidate's rotations (the barrier made x_img[1 - par] visible)
     if (threadIdx.x < ch.end - ch.begin) image_prep_one<T>(d, ch.begin + threadIdx.x, 1 - par);
-    if (threadIdx.x == 0) {
-      d.img_chunk_sum[3LL * c] = s0;
-      d.img_chunk_sum[3LL * c + 1] = s1;
-      d.img_chunk_sum[3LL * c + 2] = s2;
-    }
+    if (threadIdx.x < 3) d.img_chunk_sum[3LL * c + threadIdx.x] = tot;
   }
   if (d.fold_ctrl) {
     __shared__ int last;
