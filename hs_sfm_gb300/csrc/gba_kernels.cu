@@ -541,18 +541,29 @@ __device__ __forceinline__ void key_jacobian(const T* X, const T* IL, const T* c
   const T dcoef = cam[0] + T(2) * cam[1] * rr2 + T(3) * cam[2] * rr4;
   const T d1 = cam[3], d2 = cam[4];
   const T f = cam[5], sk = cam[6], fa = cam[5] * cam[9];
+  // (a camera without distortion adds zeros only: left out, the same values)
+  T e0[9], e1[9];
+  if (cam[0] != T(0) || cam[1] != T(0) || cam[2] != T(0) || d1 != T(0) || d2 != T(0)) {
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      const T pr2 = T(2) * (n0 * A0[j] + n1 * A1[j]);
+      const T cd = dcoef * pr2;
+      const T cross = A0[j] * n1 + A1[j] * n0;
+      e0[j] = A0[j] + (cd * n0 + coeff * A0[j]) + (T(2) * d1 * cross + d2 * (pr2 + T(4) * n0 * A0[j]));
+      e1[j] = A1[j] + (cd * n1 + coeff * A1[j]) + (T(2) * d2 * cross + d1 * (pr2 + T(4) * n1 * A1[j]));
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      e0[j] = A0[j];
+      e1[j] = A1[j];
+    }
+  }
   T out0[9], out1[9];
 #pragma unroll
   for (int j = 0; j < 9; ++j) {
-    const T pr2 = T(2) * (n0 * A0[j] + n1 * A1[j]);
-    const T cd = dcoef * pr2;
-    const T cross = A0[j] * n1 + A1[j] * n0;
-    const T e0 = A0[j] + (cd * n0 + coeff * A0[j]) +
-                 (T(2) * d1 * cross + d2 * (pr2 + T(4) * n0 * A0[j]));
-    const T e1 = A1[j] + (cd * n1 + coeff * A1[j]) +
-                 (T(2) * d2 * cross + d1 * (pr2 + T(4) * n1 * A1[j]));
-    out0[j] = f * e0 + sk * e1;
-    out1[j] = fa * e1;
+    out0[j] = f * e0[j] + sk * e1[j];
+    out1[j] = fa * e1[j];
   }
 #pragma unroll
   for (int m = 0; m < 3; ++m) { jp[m] = out0[m]; jp[3 + m] = out1[m]; }
@@ -919,9 +930,12 @@ __device__ __forceinline__ void linearize_key64(const DevPlan& d, int k, int img
   store_vec<kJRStride>(tptr_mut<double>(d.JR[par]) + (long long)kJRStride * k, rec);
 }
 
-// The records of a key chunk at parity par, one key per thread.
+// The records of a key chunk at parity par, one key per thread.  rws: the
+// weighted residuals of the chunk's keys, each written by its own thread, or
+// null: from RW.
 template <typename T>
-__device__ __forceinline__ void linearize_chunk(const DevPlan& d, const Chunk& ch, int par) {
+__device__ __forceinline__ void linearize_chunk(const DevPlan& d, const Chunk& ch, int par,
+                                                const float4* rws = nullptr) {
   const double* __restrict__ xp = d.x_pt[par];
   const T* __restrict__ rwb = tptr<T>(d.RW[par]);
   const int fix = d.prob[ch.prob].fix;
@@ -930,7 +944,12 @@ __device__ __forceinline__ void linearize_chunk(const DevPlan& d, const Chunk& c
     T cam[10];
     load_cam<T>(d, par, __ldg(d.img_cam + img), cam);
     T rw[4];
-    load_vec<4>(rwb + 4LL * k, rw);
+    if (rws) {
+      const float4 v = rws[k - ch.begin];
+      rw[0] = v.x; rw[1] = v.y; rw[2] = v.z;
+    } else {
+      load_vec<4>(rwb + 4LL * k, rw);
+    }
     if constexpr (sizeof(T) == sizeof(double)) {
       double R[12];
       load_vec<12>(d.img_rot[par] + 12LL * img, R);
@@ -1033,6 +1052,7 @@ __global__ void __launch_bounds__(256) k_cost(DevPlan d, int which) {
 // double-float, block sums in FP64.
 __global__ void __launch_bounds__(256) k_cost_ff(DevPlan d, int which) {
   __shared__ double red[32];
+  __shared__ float4 rws[kKeyChunk];   // the residuals on their way into the records
   const Chunk ch = d.key_chunks[blockIdx.x];
   const LMState& st = d.state[ch.prob];
   if (which == 0 ? !st.active : !st.evaluate) return;
@@ -1040,6 +1060,7 @@ __global__ void __launch_bounds__(256) k_cost_ff(DevPlan d, int which) {
   const float2* __restrict__ xp = d.x_ff[par];
   const float2* __restrict__ rot = d.img_rot_ff[par];
   float* __restrict__ rw = static_cast<float*>(d.RW[par]);
+  const bool records = which == 1 && d.fuse_lin, local = records && ch.end - ch.begin <= kKeyChunk;
   ff acc = {0.0f, 0.0f};
   double acc_raw = 0.0;
   for (int k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) {
@@ -1102,13 +1123,17 @@ __global__ void __launch_bounds__(256) k_cost_ff(DevPlan d, int which) {
     } else {
       acc = ff_add(acc, sqf);
     }
-    float out[4] = {e0 * sw, e1 * sw, sw, 0.0f};
-    store_vec<4>(rw + 4LL * k, out);
+    if (local) {
+      rws[k - ch.begin] = make_float4(e0 * sw, e1 * sw, sw, 0.0f);
+    } else {
+      const float out[4] = {e0 * sw, e1 * sw, sw, 0.0f};
+      store_vec<4>(rw + 4LL * k, out);
+    }
   }
   // the candidate's Jacobian records, used if it is accepted: a second pass
   // over the chunk (each thread its own keys and the residuals it just
-  // wrote), so the cost loop keeps its register count
-  if (which == 1 && d.fuse_lin) linearize_chunk<float>(d, ch, par);
+  // kept), so the cost loop keeps its register count
+  if (records) linearize_chunk<float>(d, ch, par, local ? rws : nullptr);
   double sums[2] = {double(acc.hi) + double(acc.lo), acc_raw};
   const double tot = block_sums<2>(sums, red);
   if (threadIdx.x < 2) d.key_chunk_sum[2LL * blockIdx.x + threadIdx.x] = tot;
