@@ -3760,18 +3760,38 @@ __global__ void __launch_bounds__(kCholSmallThreads, 1) k_chol_small(DevPlan d) 
 // Per problem and iteration: p.q, r.z, r.r and b.b are reduced from per-chunk
 // partials (chunks of kImageChunk images) by every CTA that needs them.
 // ---------------------------------------------------------------------------
-__device__ double block_sum_all(double v, double* smem) {
-  const double r = block_sum(v, smem);
-  if (threadIdx.x == 0) smem[32] = r;
+// Slots slot[0 .. N) of problem p's chunk partials, each summed over its chunks
+// (thread t takes chunks t, t + 256, ..., then the tree of block_sum), into
+// out[0 .. N) in every thread: one pass and two barriers for all of them (an
+// FP64 addition takes 64 cycles, and every CTA waits for these sums before
+// its own work).  red [9 N].
+template <int N>
+__device__ __forceinline__ void pcg_prob_sums(const DevPlan& d, int p, const int (&slot)[N], double* red,
+                                              double (&out)[N]) {
+  double v[N];
+#pragma unroll
+  for (int e = 0; e < N; ++e) v[e] = 0.0;
+  for (int c = d.prob_ext_chunk_off[p] + threadIdx.x; c < d.prob_ext_chunk_off[p + 1]; c += blockDim.x) {
+    const double* part = d.pcg_part + (long long)kPcgSlots * c;
+#pragma unroll
+    for (int e = 0; e < N; ++e) v[e] += part[slot[e]];
+  }
+  const double tot = block_sums<N>(v, red);
+  if (threadIdx.x < N) red[8 * N + threadIdx.x] = tot;
   __syncthreads();
-  return smem[32];
+#pragma unroll
+  for (int e = 0; e < N; ++e) out[e] = red[8 * N + e];
 }
 
-__device__ __forceinline__ double pcg_prob_sum(const DevPlan& d, int p, int slot, double* red) {
-  double v = 0.0;
-  for (int c = d.prob_ext_chunk_off[p] + threadIdx.x; c < d.prob_ext_chunk_off[p + 1]; c += blockDim.x)
-    v += d.pcg_part[(long long)kPcgSlots * c + slot];
-  return block_sum_all(v, red);
+// Six consecutive values (three 8-byte or 16-byte loads).
+template <typename T>
+__device__ __forceinline__ void load6(const T* __restrict__ p, T* o) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const auto v = reinterpret_cast<const typename Pair2<T>::type*>(p)[c];
+    o[2 * c] = v.x;
+    o[2 * c + 1] = v.y;
+  }
 }
 
 template <typename T>
@@ -3897,15 +3917,16 @@ __global__ void __launch_bounds__(256) k_pcg_init(DevPlan d) {
       rr = double(rv) * double(rv);
     }
   }
-  rz = block_sum(rz, red);
-  rr = block_sum(rr, red);
+  double sums[2] = {rz, rr};
+  const double tot = block_sums<2>(sums, red);
+  double* part = d.pcg_part + (long long)kPcgSlots * blockIdx.x;
   if (threadIdx.x == 0) {
-    double* part = d.pcg_part + (long long)kPcgSlots * blockIdx.x;
-    part[1] = rz;
-    part[3] = rr;
-    part[5] = rr;
+    part[1] = tot;
     part[6] = 0.0;
     if (blockIdx.x == d.prob_ext_chunk_off[ch.prob]) d.pcg_done[ch.prob] = 0;
+  } else if (threadIdx.x == 1) {
+    part[3] = tot;
+    part[5] = tot;
   }
 }
 
@@ -3913,7 +3934,7 @@ __global__ void __launch_bounds__(256) k_pcg_init(DevPlan d) {
 // images stored, neighbours' formed on the fly), q = S p, partial p.q.
 template <typename T>
 __global__ void __launch_bounds__(256) k_pcg_spmv(DevPlan d, int it, int loop) {
-  __shared__ double red[33];
+  __shared__ double red[9 * 4];
   // in the device-side loop `it` is the half (0, 1) of the loop body's pass
   if (loop) it += 2 * *reinterpret_cast<volatile int*>(d.pcg_it);
   if (it >= d.pcg_max_iterations) return;
@@ -3922,12 +3943,12 @@ __global__ void __launch_bounds__(256) k_pcg_spmv(DevPlan d, int it, int loop) {
   const LMState& st = d.state[p];
   if (!st.active || d.factor_flag[p] || d.pcg_done[p]) return;
   const int par = it & 1;
-  const double rz = pcg_prob_sum(d, p, 1 + par, red);
-  const double rr = pcg_prob_sum(d, p, 3 + par, red);
-  const double bb = pcg_prob_sum(d, p, 5, red);
-  if (rr <= d.pcg_tol2 * bb) return;                  // converged (or b = 0)
-  const double rzp = it > 0 ? pcg_prob_sum(d, p, 1 + (par ^ 1), red) : 1.0;
-  const T beta = it > 0 ? T(rz / rzp) : T(0);
+  // r.z, r.r, b.b and (from the second iteration on) the last r.z
+  const int slot[4] = {1 + par, 3 + par, 5, it > 0 ? 1 + (par ^ 1) : 5};
+  double sum[4];
+  pcg_prob_sums<4>(d, p, slot, red, sum);
+  if (sum[1] <= d.pcg_tol2 * sum[2]) return;          // converged (or b = 0)
+  const T beta = it > 0 ? T(sum[0] / sum[3]) : T(0);
   const T* z = tptr<T>(d.pcg_z);
   const T* pold = tptr<T>(d.pcg_p[par]);
   T* pnew = tptr_mut<T>(d.pcg_p[par ^ 1]);
@@ -3941,10 +3962,14 @@ __global__ void __launch_bounds__(256) k_pcg_spmv(DevPlan d, int it, int loop) {
     for (int e = a0 + lane; e < a1; e += 32) {
       const int2 en = __ldg(d.adj + e);
       const int j = en.y >> 1;
-      T pj[6];
+      // (the block in 16-byte loads: entry by entry, a warp's 36 loads of
+      // scattered 144-byte blocks took three quarters of the kernel)
+      T pj[6], po[6], B[36];
+      load6(z + 6LL * j, pj);
+      load6(pold + 6LL * j, po);
+      load_vec<36>(Sb + 36LL * en.x, B);
 #pragma unroll
-      for (int c = 0; c < 6; ++c) pj[c] = z[6LL * j + c] + beta * pold[6LL * j + c];
-      const T* B = Sb + 36LL * en.x;
+      for (int c = 0; c < 6; ++c) pj[c] = pj[c] + beta * po[c];
       if (!(en.y & 1)) {
 #pragma unroll
         for (int x = 0; x < 6; ++x)
@@ -3970,7 +3995,9 @@ __global__ void __launch_bounds__(256) k_pcg_spmv(DevPlan d, int it, int loop) {
       dot = double(pv) * double(qv);
     }
   }
-  dot = block_sum(dot, red);
+  __syncthreads();   // (red is read above)
+  double sums[1] = {dot};
+  dot = block_sums<1>(sums, red);
   if (threadIdx.x == 0) d.pcg_part[(long long)kPcgSlots * blockIdx.x] = dot;
 }
 
@@ -3978,7 +4005,7 @@ __global__ void __launch_bounds__(256) k_pcg_spmv(DevPlan d, int it, int loop) {
 // z = Minv r, partials of the next r.z and r.r.
 template <typename T>
 __global__ void __launch_bounds__(256) k_pcg_update(DevPlan d, int it, int loop) {
-  __shared__ double red[33];
+  __shared__ double red[9 * 4];
   if (loop) it += 2 * *reinterpret_cast<volatile int*>(d.pcg_it);
   if (it >= d.pcg_max_iterations) return;
   const Chunk ch = d.ext_chunks[blockIdx.x];
@@ -3987,9 +4014,11 @@ __global__ void __launch_bounds__(256) k_pcg_update(DevPlan d, int it, int loop)
   if (!st.active || d.factor_flag[p] || d.pcg_done[p]) return;
   const bool lead = blockIdx.x == d.prob_ext_chunk_off[p];
   const int par = it & 1;
-  const double rz = pcg_prob_sum(d, p, 1 + par, red);
-  const double rr = pcg_prob_sum(d, p, 3 + par, red);
-  const double bb = pcg_prob_sum(d, p, 5, red);
+  // r.z, r.r, b.b, p.q (the last one stale, and not looked at, once converged)
+  const int slot[4] = {1 + par, 3 + par, 5, 0};
+  double sum[4];
+  pcg_prob_sums<4>(d, p, slot, red, sum);
+  const double rz = sum[0], rr = sum[1], bb = sum[2], pq = sum[3];
   double* part = d.pcg_part + (long long)kPcgSlots * blockIdx.x;
   if (rr <= d.pcg_tol2 * bb) {
     // converged: carry this chunk's partials to the next parity so that
@@ -4001,7 +4030,6 @@ __global__ void __launch_bounds__(256) k_pcg_update(DevPlan d, int it, int loop)
     }
     return;
   }
-  const double pq = pcg_prob_sum(d, p, 0, red);
   if (!(pq > 0.0)) {
     // breakdown (the residual is at the rounding floor): keep x and stop, by
     // zeroing the next r.r, which the branch above then carries forward
@@ -4036,14 +4064,16 @@ __global__ void __launch_bounds__(256) k_pcg_update(DevPlan d, int it, int loop)
       rrn = double(rv) * double(rv);
     }
   }
-  rzn = block_sum(rzn, red);
-  rrn = block_sum(rrn, red);
-  xr = block_sum(xr, red);
+  __syncthreads();   // (red is read above)
+  double sums[3] = {rzn, rrn, xr};
+  const double tot = block_sums<3>(sums, red);
   if (threadIdx.x == 0) {
-    part[1 + (par ^ 1)] = rzn;
-    part[3 + (par ^ 1)] = rrn;
-    part[6] = xr;
+    part[1 + (par ^ 1)] = tot;
     if (lead) st.pcg_iters += 1;
+  } else if (threadIdx.x == 1) {
+    part[3 + (par ^ 1)] = tot;
+  } else if (threadIdx.x == 2) {
+    part[6] = tot;
   }
 }
 
