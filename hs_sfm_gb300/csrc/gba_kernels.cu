@@ -1839,8 +1839,9 @@ __global__ void __launch_bounds__(256) k_assemble_S(DevPlan d) {
 }
 
 // The same dense system, block by block (plans without free cameras): S is
-// zeroed first (the entries of image pairs without a common point are 0),
-// then one thread per entry of every block writes base - sum over the
+// zeroed first (the entries of image pairs without a common point are 0)
+// unless every image pair has a block (DevPlan::s_complete: nothing but the
+// blocks is read of it; one graph node of about 3 us less), then one thread per entry of every block writes base - sum over the
 // block's items (+ mu on the diagonal) exactly as k_assemble_S does, the 36
 // threads of a block reading its items' partials together; the threads of
 // row 0 of each diagonal block write the rhs.
@@ -4726,7 +4727,8 @@ int launch_assemble_S(const DevPlan& d, cudaStream_t s) {
   if (d.max_n <= 0) return 0;
   if (d.blk_prob && d.n_blocks > 0) {
     const size_t tsz = d.precision == GBA_PRECISION_MIXED ? sizeof(float) : sizeof(double);
-    if (cudaMemsetAsync(d.S, 0, size_t(d.s_elems) * tsz, s) != cudaSuccess) throw CudaError{GBA_ERR_CUDA};
+    if (!d.s_complete && cudaMemsetAsync(d.S, 0, size_t(d.s_elems) * tsz, s) != cudaSuccess)
+      throw CudaError{GBA_ERR_CUDA};
     const unsigned g = unsigned((36LL * d.n_blocks + 255) / 256);
     GBA_DISPATCH(d, (k_assemble_S_blocks<T><<<g, 256, 0, s>>>(d)));
     return 1;

@@ -1649,6 +1649,9 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
   D.items = arena.upload(items);
   D.blk_ij = arena.upload(blk_ij);
   D.s_elems = pcg ? 0 : s_off;
+  long long all_pairs = 0;
+  for (int q = 0; q < nprob; ++q) all_pairs += (long long)prob[q].num_ext * (prob[q].num_ext + 1) / 2;
+  D.s_complete = (long long)blk_ij.size() == all_pairs;
   D.blk_prob = nullptr;
   if (!pcg && !any_free && !blk_ij.empty()) {   // the dense system assembled block by block
     std::vector<int> blk_prob(blk_ij.size());
