@@ -1146,33 +1146,57 @@ __global__ void __launch_bounds__(256) k_cost_ff(DevPlan d, int which) {
   }
 }
 
-// Per point: V_p = sum J_p^T J_p, g_p = sum J_p^T r from its keys' records.
+// Keys whose products the point kernels keep in shared memory at a time (a
+// chunk of 128 points has about 700; longer ones go in parts).
+constexpr int kPointKeys = 768;
+
+// Per point: V_p = sum J_p^T J_p, g_p = sum J_p^T r from its keys' records:
+// the products a key to a thread, then added point by point in key order (as
+// the back-substitution does).
 template <typename T>
 __global__ void __launch_bounds__(kPointChunk) k_point_reduce(DevPlan d) {
+  constexpr int kCap = kPointKeys / 2;
   __shared__ unsigned long long red[2 * kPointChunk / 32];
+  __shared__ T prod[9][kCap];
   const Chunk ch = d.pt_chunks[blockIdx.x];
   const LMState& st = d.state[ch.prob];
   if (!st.relin || !st.active) return;
   const int pt = ch.begin + threadIdx.x;
   T vmax = T(0), gmax = T(0);
-  if (pt < ch.end) {
+  T V[6] = {0, 0, 0, 0, 0, 0}, g[3] = {0, 0, 0};
+  {
     const T* __restrict__ JR = tptr<T>(d.JR[st.parity]);
-    T V[6] = {0, 0, 0, 0, 0, 0}, g[3] = {0, 0, 0};
-    const int kb = __ldg(d.pt_key_off + pt), ke = __ldg(d.pt_key_off + pt + 1);
-    for (int k = kb; k < ke; ++k) {
-      T jp[8], rr[2];
-      load_vec<8>(JR + (long long)kJRStride * k, jp);
-      load_vec<2>(JR + (long long)kJRStride * k + 18, rr);
-      V[0] += jp[0] * jp[0] + jp[3] * jp[3];
-      V[1] += jp[0] * jp[1] + jp[3] * jp[4];
-      V[2] += jp[0] * jp[2] + jp[3] * jp[5];
-      V[3] += jp[1] * jp[1] + jp[4] * jp[4];
-      V[4] += jp[1] * jp[2] + jp[4] * jp[5];
-      V[5] += jp[2] * jp[2] + jp[5] * jp[5];
-      g[0] += jp[0] * rr[0] + jp[3] * rr[1];
-      g[1] += jp[1] * rr[0] + jp[4] * rr[1];
-      g[2] += jp[2] * rr[0] + jp[5] * rr[1];
+    const int k0 = __ldg(d.pt_key_off + ch.begin), k1 = __ldg(d.pt_key_off + ch.end);
+    const int kb = pt < ch.end ? __ldg(d.pt_key_off + pt) : k1, ke = pt < ch.end ? __ldg(d.pt_key_off + pt + 1) : k1;
+    for (int base = k0; base < k1; base += kCap) {
+      const int top = min(k1, base + kCap);
+      for (int k = base + int(threadIdx.x); k < top; k += kPointChunk) {
+        T jp[8], rr[2];
+        load_vec<8>(JR + (long long)kJRStride * k, jp);
+        load_vec<2>(JR + (long long)kJRStride * k + 18, rr);
+        const int e = k - base;
+        prod[0][e] = jp[0] * jp[0] + jp[3] * jp[3];
+        prod[1][e] = jp[0] * jp[1] + jp[3] * jp[4];
+        prod[2][e] = jp[0] * jp[2] + jp[3] * jp[5];
+        prod[3][e] = jp[1] * jp[1] + jp[4] * jp[4];
+        prod[4][e] = jp[1] * jp[2] + jp[4] * jp[5];
+        prod[5][e] = jp[2] * jp[2] + jp[5] * jp[5];
+        prod[6][e] = jp[0] * rr[0] + jp[3] * rr[1];
+        prod[7][e] = jp[1] * rr[0] + jp[4] * rr[1];
+        prod[8][e] = jp[2] * rr[0] + jp[5] * rr[1];
+      }
+      __syncthreads();
+      const int e1 = min(ke, top) - base;
+      for (int e = max(kb, base) - base; e < e1; ++e) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c) V[c] += prod[c][e];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) g[c] += prod[6 + c][e];
+      }
+      if (top < k1) __syncthreads();
     }
+  }
+  if (pt < ch.end) {
     if (d.pt_cons_off) {   // soft constraints: weight on the diagonal, w (x - y) in g
       const double* xp = d.x_pt[st.parity] + 3LL * pt;
       for (int c = d.pt_cons_off[pt]; c < d.pt_cons_off[pt + 1]; ++c) {
@@ -4124,6 +4148,7 @@ __global__ void k_pcg_loop_open(cudaGraphConditionalHandle h) { cudaGraphSetCond
 template <typename T>
 __global__ void __launch_bounds__(kPointChunk) k_backsub(DevPlan d) {
   __shared__ double red[32];
+  __shared__ T prod[3][kPointKeys];   // J_p^T (J_i delta_i) of the chunk's keys
   // With DevPlan::fold_ctrl the last CTA of a problem to finish runs the LM
   // step decision (k_ctrl_step's body), so every CTA of an active problem
   // arrives, also when the factorization failed and there is nothing to do.
@@ -4139,32 +4164,49 @@ __global__ void __launch_bounds__(kPointChunk) k_backsub(DevPlan d) {
     const int par = st.parity;
     const int pt = ch.begin + threadIdx.x;
     double dn2 = 0.0, xn2 = 0.0, gd = 0.0;
+    // w = sum over the point's keys of J_p^T (J_i delta_i) from the Jacobian
+    // records, then t = C^-1 (g - w) with C^-1 g = h.  The products are formed
+    // a key to a thread (the chunk's records are consecutive, every lane has a
+    // key, no load waits for another key's) and added point by point, in key
+    // order, from shared memory.  A point to a thread throughout, a warp
+    // walked its longest track, two dependent loads a key: 512 windows 764 us.
+    T w0 = T(0), w1 = T(0), w2 = T(0);
+    {
+      const T* __restrict__ JR = tptr<T>(d.JR[par]);
+      const T* __restrict__ delta = tptr<T>(d.b);
+      const int k0 = __ldg(d.pt_key_off + ch.begin), k1 = __ldg(d.pt_key_off + ch.end);
+      const int kb = pt < ch.end ? __ldg(d.pt_key_off + pt) : k1, ke = pt < ch.end ? __ldg(d.pt_key_off + pt + 1) : k1;
+      for (int base = k0; base < k1; base += kPointKeys) {
+        const int top = min(k1, base + kPointKeys);
+        for (int k = base + int(threadIdx.x); k < top; k += kPointChunk) {
+          T rec[kJRStride], dl[6];
+          load_vec<kJRStride>(JR + (long long)kJRStride * k, rec);
+          const int ext = d.img_ext ? __ldg(d.img_ext + __ldg(d.key_img + k)) : __ldg(d.key_img + k);
+          load6(delta + 6LL * ext, dl);
+          T u0 = T(0), u1 = T(0);
+#pragma unroll
+          for (int c = 0; c < 6; ++c) {
+            u0 += rec[6 + c] * dl[c];
+            u1 += rec[12 + c] * dl[c];
+          }
+          prod[0][k - base] = rec[0] * u0 + rec[3] * u1;
+          prod[1][k - base] = rec[1] * u0 + rec[4] * u1;
+          prod[2][k - base] = rec[2] * u0 + rec[5] * u1;
+        }
+        __syncthreads();
+        const int e1 = min(ke, top) - base;
+        for (int e = max(kb, base) - base; e < e1; ++e) {
+          w0 += prod[0][e];
+          w1 += prod[1][e];
+          w2 += prod[2][e];
+        }
+        if (top < k1) __syncthreads();   // (before the next part overwrites them)
+      }
+    }
     if (pt < ch.end) {
       T ps[12];
       load_vec<12>(tptr<T>(d.PS) + 12LL * pt, ps);
       const T i00 = ps[0], m10 = ps[1], i11 = ps[2], m20 = ps[3], m21 = ps[4], i22 = ps[5];
-      const T* __restrict__ JR = tptr<T>(d.JR[st.parity]);
-      const int kb = __ldg(d.pt_key_off + pt), ke = __ldg(d.pt_key_off + pt + 1);
-      // w = sum over the point's keys of J_p^T (J_i delta_i) from the
-      // Jacobian records (the point's keys are consecutive), then
-      // t = C^-1 (g - w) with C^-1 g = h
-      T w0 = T(0), w1 = T(0), w2 = T(0);
-      for (int k = kb; k < ke; ++k) {
-        T rec[kJRStride];
-        load_vec<kJRStride>(JR + (long long)kJRStride * k, rec);
-        const int ext = d.img_ext ? __ldg(d.img_ext + __ldg(d.key_img + k)) : __ldg(d.key_img + k);
-        const T* di = tptr<T>(d.b) + 6LL * ext;
-        T u0 = T(0), u1 = T(0);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-          const T dl = di[c];
-          u0 += rec[6 + c] * dl;
-          u1 += rec[12 + c] * dl;
-        }
-        w0 += rec[0] * u0 + rec[3] * u1;
-        w1 += rec[1] * u0 + rec[4] * u1;
-        w2 += rec[2] * u0 + rec[5] * u1;
-      }
       T t0 = ps[6] - i00 * w0, t1 = ps[7] - (m10 * w0 + i11 * w1), t2 = ps[8] - (m20 * w0 + m21 * w1 + i22 * w2);
       // free cameras: the point's camera records (Z = C^-1 W) against their
       // reduced-system images' deltas
