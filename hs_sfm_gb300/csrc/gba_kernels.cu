@@ -581,7 +581,11 @@ __device__ __forceinline__ void load_cam(const DevPlan& d, int par, int cam, T* 
 template <>
 __device__ __forceinline__ void load_cam<float>(const DevPlan& d, int par, int cam, float* out) {
 #pragma unroll
-  for (int j = 0; j < 10; ++j) out[j] = d.cam32[par][10 * cam + j];
+  for (int j = 0; j < 5; ++j) {
+    const float2 v = __ldg(reinterpret_cast<const float2*>(d.cam32[par] + 10LL * cam) + j);
+    out[2 * j] = v.x;
+    out[2 * j + 1] = v.y;
+  }
 }
 template <>
 __device__ __forceinline__ void load_cam<double>(const DevPlan& d, int par, int cam, double* out) {
@@ -833,8 +837,31 @@ __global__ void __launch_bounds__(256) k_cons_cost(DevPlan d, int which) {
 __device__ __forceinline__ float whiten_u(float l00, float a, float l10, float b) { return l00 * a + l10 * b; }
 __device__ __forceinline__ double whiten_u(double l00, double a, double l10, double b) { return fma(l00, a, l10 * b); }
 
+// FP32 records (80 bytes: five 16-byte words) of a warp's keys on their way to
+// memory: each lane puts its own into its slot, and the warp writes the slots
+// word by word to consecutive addresses, whole sectors.  A record to a lane,
+// every store instruction left 32 half-written sectors 80 bytes apart (the
+// free-camera grid with its two records a key: 70 -> 61 us).  The odd pitch
+// keeps both sides free of bank conflicts.  Reading records this way was
+// slower (point sums of 512 windows 477 -> 610 us): L1 holds the lines between
+// a lane's five loads, and shared memory and registers cost warps.
+constexpr int kRecWords = kJRStride * int(sizeof(float)) / 16;
+using RecordSlots = uint4[32 * kRecWords];
+
+// The first n slots to the records of keys k, k + 1, ...
+__device__ __forceinline__ void store_record_slots(float* recs, long long k, int n, const RecordSlots& slots, int lane) {
+  uint4* w = reinterpret_cast<uint4*>(recs) + kRecWords * k;
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < kRecWords; ++u) {
+    const int c = lane + 32 * u;
+    if (c < kRecWords * n) w[c] = slots[c];
+  }
+  __syncwarp();
+}
+
 template <typename T>
-__device__ __forceinline__ void linearize_cam(const DevPlan& d, int k, int par, T* jc, T sw) {
+__device__ __forceinline__ void linearize_cam(const DevPlan& d, int k, T* jc, T sw, T* out) {
   T l00 = T(1), l10 = T(0), l11 = T(1);
   if (d.key_wl) {
     l00 = T(__ldg(d.key_wl + 3LL * k));
@@ -847,11 +874,14 @@ __device__ __forceinline__ void linearize_cam(const DevPlan& d, int k, int par, 
     jc[m] = whiten_u(l00, a, l10, b) * sw;
     jc[10 + m] = l11 * b * sw;
   }
-  store_vec<20>(tptr_mut<T>(d.JC[par]) + 20LL * k, jc);
+  store_vec<20>(out, jc);
 }
 
+// The FP32 records of a warp's keys k0 .. k0 + n - 1 (this lane's: k).
 __device__ __forceinline__ void linearize_key(const DevPlan& d, int k, int par, int fix, const float* X,
-                                              const float* il, const float* cam, float rw0, float rw1, float sw) {
+                                              const float* il, const float* cam, float rw0, float rw1, float sw,
+                                              RecordSlots& slots, int lane, int k0, int n) {
+  float* const own = reinterpret_cast<float*>(slots + lane * kRecWords);
   float jp[6], ji[12], nrm[2];
   key_jacobian<float>(X, il, cam, jp, ji, nrm);
   if (fix & 1) {   // fixed points: no point columns
@@ -865,7 +895,8 @@ __device__ __forceinline__ void linearize_key(const DevPlan& d, int k, int par, 
   if (d.free_cams) {
     float jc[20];
     camera_jacobian<float>(nrm[0], nrm[1], cam, jc);
-    linearize_cam<float>(d, k, par, jc, sw);
+    linearize_cam<float>(d, k, jc, sw, own);
+    store_record_slots(tptr_mut<float>(d.JC[par]), k0, n, slots, lane);   // (20 values too)
   }
   if (d.key_wl) {
     const float l00 = float(__ldg(d.key_wl + 3LL * k)), l10 = float(__ldg(d.key_wl + 3LL * k + 1)),
@@ -895,7 +926,8 @@ __device__ __forceinline__ void linearize_key(const DevPlan& d, int k, int par, 
   for (int m = 0; m < 12; ++m) rec[6 + m] = ji[m];
   rec[18] = rw0;
   rec[19] = rw1;
-  store_vec<kJRStride>(tptr_mut<float>(d.JR[par]) + (long long)kJRStride * k, rec);
+  store_vec<kJRStride>(own, rec);
+  store_record_slots(tptr_mut<float>(d.JR[par]), k0, n, slots, lane);
 }
 
 // The FP64 record of key k from its projection p and the rotation R of its image.
@@ -923,7 +955,7 @@ __device__ __forceinline__ void linearize_key64(const DevPlan& d, int k, int img
   if (d.free_cams) {
     double jc[20];
     camera_jacobian64(p, cam, jc);
-    linearize_cam<double>(d, k, par, jc, sw);
+    linearize_cam<double>(d, k, jc, sw, tptr_mut<double>(d.JC[par]) + 20LL * k);
   }
   rec[18] = rw0;
   rec[19] = rw1;
@@ -939,26 +971,21 @@ __device__ __forceinline__ void linearize_chunk(const DevPlan& d, const Chunk& c
   const double* __restrict__ xp = d.x_pt[par];
   const T* __restrict__ rwb = tptr<T>(d.RW[par]);
   const int fix = d.prob[ch.prob].fix;
-  for (int k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) {
-    const int img = __ldg(d.key_img + k), pt = __ldg(d.key_pt + k);
-    T cam[10];
-    load_cam<T>(d, par, __ldg(d.img_cam + img), cam);
-    T rw[4];
-    if (rws) {
-      const float4 v = rws[k - ch.begin];
-      rw[0] = v.x; rw[1] = v.y; rw[2] = v.z;
-    } else {
-      load_vec<4>(rwb + 4LL * k, rw);
-    }
-    if constexpr (sizeof(T) == sizeof(double)) {
-      double R[12];
-      load_vec<12>(d.img_rot[par] + 12LL * img, R);
-      const double X[3] = {xp[3LL * pt], xp[3LL * pt + 1], xp[3LL * pt + 2]};
-      Proj64 p;
-      project64(R, X, cam, p);
-      linearize_key64(d, k, img, par, fix, R, cam, p, rw[0], rw[1], rw[2]);
-    } else {
-      float X[3], il[12];
+  if constexpr (sizeof(T) == sizeof(float)) {
+    __shared__ RecordSlots recs[256 / 32];   // (launched with 256 threads)
+    const int lane = threadIdx.x & 31;
+    __syncwarp();   // (rws)
+    for (int k0 = ch.begin + int(threadIdx.x) - lane; k0 < ch.end; k0 += blockDim.x) {
+      const int k = min(k0 + lane, ch.end - 1);   // (the last key again where there is none)
+      const int img = __ldg(d.key_img + k), pt = __ldg(d.key_pt + k);
+      float cam[10], rw[4], X[3], il[12];
+      load_cam<float>(d, par, __ldg(d.img_cam + img), cam);
+      if (rws) {
+        const float4 v = rws[k - ch.begin];
+        rw[0] = v.x; rw[1] = v.y; rw[2] = v.z;
+      } else {
+        load_vec<4>(rwb + 4LL * k, rw);
+      }
       if (d.x_ff[par]) {   // mixed: high part of the mirror
         const float2* xf = d.x_ff[par] + 3LL * pt;
         X[0] = xf[0].x; X[1] = xf[1].x; X[2] = xf[2].x;
@@ -966,7 +993,22 @@ __device__ __forceinline__ void linearize_chunk(const DevPlan& d, const Chunk& c
         X[0] = float(xp[3LL * pt]); X[1] = float(xp[3LL * pt + 1]); X[2] = float(xp[3LL * pt + 2]);
       }
       load_vec<12>(tptr<float>(d.img_lin[par]) + 12LL * img, il);
-      linearize_key(d, k, par, fix, X, il, cam, rw[0], rw[1], rw[2]);
+      linearize_key(d, k, par, fix, X, il, cam, rw[0], rw[1], rw[2], recs[threadIdx.x >> 5], lane, k0,
+                    min(32, ch.end - k0));
+    }
+  } else {
+    for (int k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) {
+      const int img = __ldg(d.key_img + k), pt = __ldg(d.key_pt + k);
+      T cam[10];
+      load_cam<T>(d, par, __ldg(d.img_cam + img), cam);
+      T rw[4];
+      load_vec<4>(rwb + 4LL * k, rw);
+      double R[12];
+      load_vec<12>(d.img_rot[par] + 12LL * img, R);
+      const double X[3] = {xp[3LL * pt], xp[3LL * pt + 1], xp[3LL * pt + 2]};
+      Proj64 p;
+      project64(R, X, cam, p);
+      linearize_key64(d, k, img, par, fix, R, cam, p, rw[0], rw[1], rw[2]);
     }
   }
 }
@@ -1049,8 +1091,14 @@ __global__ void __launch_bounds__(256) k_cost(DevPlan d, int which) {
 
 // Mixed-path cost: the projection in double-float from the double-float
 // mirrors of x, R|t, the keys and the cameras; per-thread sums in
-// double-float, block sums in FP64.
-__global__ void __launch_bounds__(256) k_cost_ff(DevPlan d, int which) {
+// double-float, block sums in FP64.  Bound by its instructions and by L1 (55%
+// and 71% busy, 32 warps an SM): the keys of a warp see many images, so every
+// load instruction of an image's values is some 20 lines.  R|t, the camera and
+// the key come in 16-byte loads (half as many), which with the records' store
+// (store_record_slots) took 512 windows from 1117 to 1012 us, the random walk
+// from 485 to 420, the grid from 60.6 to 53.0 and its free cameras from 76 to
+// 61.  Without the bound of 64 registers: 80, three blocks an SM, 1249 us.
+__global__ void __launch_bounds__(256, 4) k_cost_ff(DevPlan d, int which) {
   __shared__ double red[32];
   __shared__ float4 rws[kKeyChunk];   // the residuals on their way into the records
   const Chunk ch = d.key_chunks[blockIdx.x];
@@ -1065,21 +1113,24 @@ __global__ void __launch_bounds__(256) k_cost_ff(DevPlan d, int which) {
   double acc_raw = 0.0;
   for (int k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) {
     const int img = __ldg(d.key_img + k), pt = __ldg(d.key_pt + k);
-    const float2* R = rot + 12LL * img;
+    float R[24];
+    load_vec<24>(reinterpret_cast<const float*>(rot + 12LL * img), R);
+    auto Rm = [&](int m) { return ff{R[2 * m], R[2 * m + 1]}; };
     const ff X0 = ff_ld(xp[3LL * pt]), X1 = ff_ld(xp[3LL * pt + 1]), X2 = ff_ld(xp[3LL * pt + 2]);
     ff y[3];
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-      ff a = ff_ld(R[9 + m]);
-      a = ff_fma(ff_ld(R[3 * m]), X0, a);
-      a = ff_fma(ff_ld(R[3 * m + 1]), X1, a);
-      y[m] = ff_fma(ff_ld(R[3 * m + 2]), X2, a);
+      ff a = Rm(9 + m);
+      a = ff_fma(Rm(3 * m), X0, a);
+      a = ff_fma(Rm(3 * m + 1), X1, a);
+      y[m] = ff_fma(Rm(3 * m + 2), X2, a);
     }
     const ff iz = ff_rcp(y[2]);
     ff n0 = ff_mul(y[0], iz), n1 = ff_mul(y[1], iz);
-    const float2* cam = d.cam_ff[par] + 10 * __ldg(d.img_cam + img);
-    const ff k1 = ff_ld(cam[0]), k2 = ff_ld(cam[1]), k3 = ff_ld(cam[2]);
-    const ff d1 = ff_ld(cam[3]), d2 = ff_ld(cam[4]);
+    const float4* cam = reinterpret_cast<const float4*>(d.cam_ff[par] + 10 * __ldg(d.img_cam + img));
+    const float4 cam01 = __ldg(cam), cam23 = __ldg(cam + 1), cam45 = __ldg(cam + 2);
+    const ff k1 = {cam01.x, cam01.y}, k2 = {cam01.z, cam01.w}, k3 = {cam23.x, cam23.y};
+    const ff d1 = {cam23.z, cam23.w}, d2 = {cam45.x, cam45.y};
     const ff r2 = ff_add(ff_mul(n0, n0), ff_mul(n1, n1));
     ff dx = {0.0f, 0.0f}, dy = {0.0f, 0.0f};
     if (k1.hi != 0.0f || k2.hi != 0.0f || k3.hi != 0.0f) {
@@ -1094,12 +1145,13 @@ __global__ void __launch_bounds__(256) k_cost_ff(DevPlan d, int which) {
     }
     n0 = ff_add(n0, dx);
     n1 = ff_add(n1, dy);
-    const ff f = ff_ld(cam[5]), sk = ff_ld(cam[6]), cx = ff_ld(cam[7]), cy = ff_ld(cam[8]);
-    const ff fa = ff_ld(cam[9]);   // f * a, stored pre-multiplied
+    const float4 cam67 = __ldg(cam + 3), cam89 = __ldg(cam + 4);
+    const ff f = {cam45.z, cam45.w}, sk = {cam67.x, cam67.y}, cx = {cam67.z, cam67.w}, cy = {cam89.x, cam89.y};
+    const ff fa = {cam89.z, cam89.w};   // f * a, stored pre-multiplied
     const ff u = ff_add(ff_fma(f, n0, ff_mul(sk, n1)), cx);
     const ff v = ff_fma(fa, n1, cy);
-    const float2 ob0 = d.key_obs_ff[2LL * k], ob1 = d.key_obs_ff[2LL * k + 1];
-    ff e0f = ff_add(u, ff_neg(ff_ld(ob0))), e1f = ff_add(v, ff_neg(ff_ld(ob1)));   // r = f(x) - y
+    const float4 ob = __ldg(reinterpret_cast<const float4*>(d.key_obs_ff + 2LL * k));
+    ff e0f = ff_add(u, ff_neg(ff{ob.x, ob.y})), e1f = ff_add(v, ff_neg(ff{ob.z, ob.w}));   // r = f(x) - y
     {
       const float r0 = e0f.hi + e0f.lo, r1 = e1f.hi + e1f.lo;
       acc_raw += double(fmaf(r0, r0, r1 * r1));
@@ -1152,9 +1204,11 @@ constexpr int kPointKeys = 768;
 
 // Per point: V_p = sum J_p^T J_p, g_p = sum J_p^T r from its keys' records:
 // the products a key to a thread, then added point by point in key order (as
-// the back-substitution does).
+// the back-substitution does).  FP32: bound by DRAM (68%) and by the loads in
+// flight, so 48 registers for ten blocks an SM (512 windows 477 -> 460 us; 40
+// and twelve blocks spill: 495).
 template <typename T>
-__global__ void __launch_bounds__(kPointChunk) k_point_reduce(DevPlan d) {
+__global__ void __launch_bounds__(kPointChunk, sizeof(T) == sizeof(float) ? 10 : 0) k_point_reduce(DevPlan d) {
   constexpr int kCap = kPointKeys / 2;
   __shared__ unsigned long long red[2 * kPointChunk / 32];
   __shared__ T prod[9][kCap];
@@ -4146,7 +4200,7 @@ __global__ void k_pcg_loop_open(cudaGraphConditionalHandle h) { cudaGraphSetCond
 // back-substitution and update
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(kPointChunk) k_backsub(DevPlan d) {
+__global__ void __launch_bounds__(kPointChunk, sizeof(T) == sizeof(float) ? 10 : 0) k_backsub(DevPlan d) {
   __shared__ double red[32];
   __shared__ T prod[3][kPointKeys];   // J_p^T (J_i delta_i) of the chunk's keys
   // With DevPlan::fold_ctrl the last CTA of a problem to finish runs the LM
@@ -4169,7 +4223,10 @@ __global__ void __launch_bounds__(kPointChunk) k_backsub(DevPlan d) {
     // a key to a thread (the chunk's records are consecutive, every lane has a
     // key, no load waits for another key's) and added point by point, in key
     // order, from shared memory.  A point to a thread throughout, a warp
-    // walked its longest track, two dependent loads a key: 512 windows 764 us.
+    // walked its longest track, two dependent loads a key: 512 windows 764 us
+    // instead of 647, random walk 349 instead of 239.  The loads' latency
+    // bounds it (DRAM 48% busy at 29 warps an SM), so FP32 is held to 48
+    // registers for 40 warps: 586 and 228 us.
     T w0 = T(0), w1 = T(0), w2 = T(0);
     {
       const T* __restrict__ JR = tptr<T>(d.JR[par]);
