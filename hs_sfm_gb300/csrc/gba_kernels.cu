@@ -15,15 +15,15 @@
 //                     normal_equation_builder.hpp:207-220,377-391)
 //   k_image_reduce   per image: U_i = sum J_i^T J_i, g_i = sum J_i^T r with
 //                    compensated (Kahan) lane sums (normal_equation_builder.hpp:221-234)
-//   k_point_schur    per point: C C^T = V_p + mu I, Z_a = C^-1 J_p^T J_i,
-//                    h_p = C^-1 g_p (normal_equation_solver.hpp:141-184)
+//   k_point_factor   per point: C C^T = V_p + mu I, h_p = C^-1 g_p, and
+//   k_key_z          per key: Z_a = C^-1 J_p^T J_i (normal_equation_solver.hpp:141-184)
 //   k_assemble_items per block (i<=j) of the reduced system: -sum Z_a^T Z_b
 //                    over the points seen by both images, rhs terms
 //                    (normal_equation_solver.hpp:190-267,398-420)
 //   k_assemble_S     dense reduced system S and rhs b (T), block sums in FP64
 //   k_chol_*         tiled Cholesky (T) with the forward solve folded in,
 //                    then the backward solve (normal_equation_solver.hpp:448-466)
-//   k_backsub        delta_p = C^-T (h_p - sum Z_a delta_i), x_new = x - delta,
+//   k_backsub        delta_p = C^-T (h_p - C^-1 sum J_p^T J_i delta_i), x_new = x - delta,
 //                    and the candidate's image rotations
 //                    (normal_equation_solver.hpp:468-538)
 //   k_ctrl_*         the LM decisions per problem on the device (Madsen,
@@ -2310,17 +2310,21 @@ __device__ __forceinline__ int ld_acquire_shared(const int* p) {
 // the next pair's two columns are updated and its pivot block read first, the
 // half's other columns (from the published ones, four to a load) fill the
 // latency of the next square roots.  The waits (for `step`, which its owner
-// always reaches) are bounded all the same.  1,330 cycles; all 32 columns in
-// one warp took 2,630 (its issue slots), over four warps with a barrier a pair
-// (the FP64 form) 4,400.
-template <int B>
-__device__ __forceinline__ void potrf_half(float (&a)[kTile / 2], PotrfBuf<float>& fb, int lane, bool& ok) {
+// always reaches) are bounded all the same.  In a loop 1,330 cycles; all 32
+// columns in one warp took 2,630 (its issue slots), over four warps with a
+// barrier a pair (the FP64 form) 4,400.  In the factorization's chain, where
+// an SM runs it the second time only, 1.86 us (3,500 cycles).  Both halves run
+// the same instructions (B at run time) and warp 2 applies the first half's
+// pairs in a loop: 512 small systems, each a CTA's only factorization, 161 ->
+// 148 us against a copy of the code per half.
+__device__ __forceinline__ void potrf_half(float (&a)[kTile / 2], int B, PotrfBuf<float>& fb, int lane, bool& ok) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int H = kTile / 2;
   float p0 = __shfl_sync(FULL, a[0], B), p1 = __shfl_sync(FULL, a[0], B + 1), p2 = __shfl_sync(FULL, a[1], B + 1);
   // every column index is a compile-time constant, so a[] stays in registers
   static_for<0, H, 2>([&](auto hc) {
-    constexpr int h = decltype(hc)::value, j = B + h, s = j / 2;
+    constexpr int h = decltype(hc)::value;
+    const int j = B + h, s = j / 2;
     const float det = fmaf(p0, p2, -(p1 * p1));
     const float r0 = rsqrtf(p0), rd = rsqrtf(det);
     const float l00 = p0 * r0;             // sqrt(p0)
@@ -2366,11 +2370,9 @@ __device__ __forceinline__ bool tile_potrf_inverse(const Tile<float>& D, Tile<fl
     float a[H];
 #pragma unroll
     for (int q = 0; q < H; q += 4) load16(&D[lane][(warp == 0 ? 0 : H) + q], a + q);
-    if (warp == 0) {
-      potrf_half<0>(a, fb, lane, ok);
-    } else {
-      static_for<0, H / 2, 1>([&](auto sc) {
-        constexpr int s = decltype(sc)::value;
+    if (warp == 2) {
+#pragma unroll 1
+      for (int s = 0; s < H / 2; ++s) {
         wait_step(s);
         const float li0 = fb.f[s][0][lane], li1 = fb.f[s][1][lane];
 #pragma unroll
@@ -2381,9 +2383,9 @@ __device__ __forceinline__ bool tile_potrf_inverse(const Tile<float>& D, Tile<fl
 #pragma unroll
           for (int e = 0; e < 4; ++e) a[l + e] = fmaf(-li1, c1[e], fmaf(-li0, c0[e], a[l + e]));
         }
-      });
-      potrf_half<H>(a, fb, lane, ok);
+      }
     }
+    potrf_half(a, warp == 0 ? 0 : H, fb, lane, ok);
   } else if (warp == 1) {
     float x[kTile];
 #pragma unroll
