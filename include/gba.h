@@ -181,12 +181,14 @@ typedef struct gba_options {
    * camera_shared_ceres_optimizor.hpp:478); 0 disables the test. */
   double function_tolerance;
   /* Work-item sizes of the two reductions split into per-warp items: key
-   * pairs per Schur-assembly item (0: 1024) and keys per image-reduction
-   * item (0: 512).  They change the grouping (and so the rounding) of the
+   * pairs per Schur-assembly item (0: mixed 1024, FP64 by the problem's
+   * size, at most 1024) and keys per image-reduction item (0: mixed 512,
+   * FP64 by the problem's size, at most 256).  They change the grouping (and so the rounding) of the
    * block sums, not the model; gba_autotune picks them for a batch. */
   int32_t pair_item;
   int32_t image_item;
-  /* Keys per key work chunk (0: 1024): the unit of the cost, Jacobian and
+  /* Keys per key work chunk (0: mixed 1024, FP64 by the problem's size, at
+   * most 1024): the unit of the cost, Jacobian and
    * Z kernels and of the cost's partial sums (so it changes the rounding of
    * the cost sum, not the model); gba_autotune picks it with the others. */
   int32_t key_item;
@@ -213,8 +215,7 @@ typedef struct gba_tuning {
   int32_t pair_item;
   int32_t image_item;
   double ms_per_iteration;           /* the chosen item sizes              */
-  double default_ms_per_iteration;   /* pair_item 1024, image_item 512,
-                                        key_item 1024                      */
+  double default_ms_per_iteration;   /* with the sizes of option 0            */
   int32_t candidates;                /* configurations timed               */
   int32_t key_item;
   int32_t z_layout;                  /* GBA_Z_RECORDS or GBA_Z_PLANES      */
