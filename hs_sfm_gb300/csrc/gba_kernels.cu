@@ -3707,7 +3707,7 @@ __global__ void __launch_bounds__(256) k_chol_solve_small(DevPlan d) {
 // per-element arithmetic is that of k_chol_step, so the bits are those of
 // k_chol_step and k_chol_dataflow; then the backward solve of
 // k_chol_solve_small.  With two groups, one after the other through every
-// phase, 512 windows took 192 us an iteration.
+// phase, 512 windows took 192 us an iteration instead of 148.
 constexpr int kCholSmallThreads = 512;
 
 template <typename T>
