@@ -34,6 +34,8 @@ constexpr double kZPlanesDensity = 0.2;
 // Plans with at least this many keys fork each LM iteration (two streams)
 constexpr long long kForkMinKeys = 300000;
 constexpr int kItemStride = 44;    // per work item: 36 block + 6 rhs + pad
+template <typename T>
+constexpr long long kImageItemStride = sizeof(T) == sizeof(float) ? 28 : 56;   // per image item: the 27 sums, FP64 twice
 
 // Work-item sizes left to the library (option 0).  The mixed path keeps fixed
 // sizes: the grouping of its FP32 sums is part of its results.  The FP64 path
@@ -137,7 +139,7 @@ struct DevPlan {
   int n_img_items;
   const int4* img_items;     // (image, q begin, q end, prob), <= kImageItem keys
   const int* img_item_off;   // [I+1] items of each image
-  double* img_item_partial;  // [items * 28]
+  double* img_item_partial;  // [items * kImageItemStride]: the 27 sums, FP64 also what they lack (from 28)
   double* cam64[2];          // [C*10]  k1 k2 k3 d1 d2 f s cx cy a, by parity
   float* cam32[2];           // [C*10]  (both parities the same array while cameras are fixed)
   // parameters (double buffered by LMState::parity)

@@ -159,13 +159,14 @@ __host__ __device__ constexpr int warp_scatter_max(int n) {
   for (int o = 16; o > 0; o >>= 1) n = (n + 1) / 2;
   return n;
 }
-template <int N, int O = 16, typename T>
+// kLast: the levels below it are left to the caller.
+template <int N, int O = 16, int kLast = 1, typename T>
 __device__ __forceinline__ void warp_scatter_sums(T* v, int lane, int& base, int& count) {
   if constexpr (O == 16) {
     base = 0;
     count = N;
   }
-  if constexpr (O > 0) {
+  if constexpr (O >= kLast) {
     constexpr int H = (N + 1) / 2;
     const bool up = (lane & O) != 0;
 #pragma unroll
@@ -176,7 +177,7 @@ __device__ __forceinline__ void warp_scatter_sums(T* v, int lane, int& base, int
     }
     base += up ? H : 0;
     count = up ? count - H : min(count, H);
-    warp_scatter_sums<H, O / 2, T>(v, lane, base, count);
+    warp_scatter_sums<H, O / 2, kLast, T>(v, lane, base, count);
   }
 }
 
@@ -1290,14 +1291,28 @@ __global__ void __launch_bounds__(kPointChunk, sizeof(T) == sizeof(float) ? 10 :
 }
 
 // image reduce: U_i = sum J_i^T J_i, g_i = sum J_i^T r.  Each image's keys
-// are split into work items (one warp each); k_image_finalize adds an image's
-// items in FP64.  The FP32 lanes add with Kahan compensation (up to 16 keys a
-// lane).  The FP64 lanes add plain FMA chains of at most eight keys: the pipe
-// takes 64 cycles an instruction, Kahan sums took three times as many, and
-// with four interleaved sums over the items the error against exact sums
-// is no larger (500 to 20,000 keys: 5.1e-17 to 6.3e-17 of the sum of
-// magnitudes, before 5.3e-17 to 1.1e-16, root mean square).
+// are split into work items (one warp each) whose lanes add with
+// compensation; k_image_finalize adds an image's items in FP64.
+//
+// FP32: Kahan, its order of operations part of the mixed path's results.
+// FP64 (the pipe takes 64 cycles an instruction): the compensation enters the
+// products' FMA chain, and a lane's keys are taken two to a compensated
+// addition (3.5 instructions a key and entry instead of Kahan's 6), the carry
+// register holding the first key's products; every key is folded in items
+// of more than 256 keys (a caller's image_item) and in an image's only item.
+// The tree's last addition keeps its rounding error, which k_image_finalize
+// adds again.  Error against exact sums, root mean square relative to the sum
+// of magnitudes (Kahan lanes over 512-key items added in order in
+// parentheses): signed terms, 500 keys an image 6.8e-18 (7.1e-18), 5,000
+// 2.2e-18 (2.9e-18), 20,000 1.1e-18 (2.1e-18); positive terms 5.0e-17
+// (7.1e-17), 5.3e-17 (1.1e-16), 5.3e-17 (1.9e-16).  Plain FMA chains were as
+// good for positive terms but up to 20% (default items) and 3.6 times
+// (4,096-key items) worse for signed ones; the compensation takes 24 FP64
+// windows from 19.1 to 19.6 ms a solve of 12 iterations.
 // ---------------------------------------------------------------------------
+enum AddMode { kAddChain, kAddFirst, kAddFold };   // FP64: carry on, start the sum, fold into it
+
+template <AddMode kMode>
 __device__ __forceinline__ void add_dot2(float& acc, float& cmp, float x0, float y0, float x1, float y1) {
   const float term = x0 * y0 + x1 * y1;
   const float y = term - cmp;
@@ -1305,8 +1320,44 @@ __device__ __forceinline__ void add_dot2(float& acc, float& cmp, float x0, float
   cmp = (t - acc) - y;
   acc = t;
 }
-__device__ __forceinline__ void add_dot2(double& acc, double&, double x0, double y0, double x1, double y1) {
-  acc = fma(x1, y1, fma(x0, y0, acc));
+// (cmp: what acc lacks, to be added)
+template <AddMode kMode>
+__device__ __forceinline__ void add_dot2(double& acc, double& cmp, double x0, double y0, double x1, double y1) {
+  const double y = fma(x1, y1, fma(x0, y0, cmp));
+  if constexpr (kMode == kAddFold) {
+    const double t = acc + y;
+    cmp = y - (t - acc);
+    acc = t;
+  } else if constexpr (kMode == kAddFirst) {   // (acc is 0: the same)
+    acc = y;
+    cmp = 0.0;
+  } else {
+    cmp = y;
+  }
+}
+// a + b = s + e exactly
+__device__ __forceinline__ double two_sum(double a, double b, double& e) {
+  const double s = a + b, bb = s - a;
+  e = (a - (s - bb)) + (b - bb);
+  return s;
+}
+
+// One key's products into the 27 sums; v: its record from value 4 on.
+template <AddMode kMode, typename T>
+__device__ __forceinline__ void add_image_key(T* acc, T* cmp, const T* v) {
+  const T* ji = v + 2;
+  const T r0 = v[14], r1 = v[15];
+  int e = 0;
+#pragma unroll
+  for (int a = 0; a < 6; ++a) {
+#pragma unroll
+    for (int b = a; b < 6; ++b) {
+      add_dot2<kMode>(acc[e], cmp[e], ji[a], ji[b], ji[6 + a], ji[6 + b]);
+      ++e;
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 6; ++a) add_dot2<kMode>(acc[21 + a], cmp[21 + a], ji[a], r0, ji[6 + a], r1);
 }
 
 template <typename T>
@@ -1318,7 +1369,7 @@ __global__ void __launch_bounds__(256) k_image_reduce(DevPlan d) {
   const LMState& st = d.state[it.w];
   if (!st.relin || !st.active) return;
   const T* __restrict__ JR = tptr<T>(d.JR[st.parity]);
-  T acc[27], cmp[27];   // (cmp: FP32 only)
+  T acc[27], cmp[27];
 #pragma unroll
   for (int e = 0; e < 27; ++e) { acc[e] = T(0); cmp[e] = T(0); }
   // two loads deep: the key two rounds ahead and the record of the next round
@@ -1331,33 +1382,51 @@ __global__ void __launch_bounds__(256) k_image_reduce(DevPlan d) {
   int kn = q < it.z ? __ldg(d.img_keys + q) : 0;
   if (q < it.z) load_vec<kUse>(JR + (long long)kJRStride * kn + 4, next);
   kn = q + 32 < it.z ? __ldg(d.img_keys + q + 32) : kn;
+  // (FP64) fold every key: long lanes, and an image's only item
+  const bool whole = it.z - it.y > 256 || __ldg(d.img_item_off + it.x + 1) - __ldg(d.img_item_off + it.x) == 1;
+  bool chain = false, first = true;   // the last key's products wait in cmp; no sum yet
   for (; q < it.z; q += 32) {
     T rec[kUse];
 #pragma unroll
     for (int e = 0; e < kUse; ++e) rec[e] = next[e];
     if (q + 32 < it.z) load_vec<kUse>(JR + (long long)kJRStride * kn + 4, next);
     if (q + 64 < it.z) kn = __ldg(d.img_keys + q + 64);
-    const T* ji = rec + 2;
-    const T r0 = rec[14], r1 = rec[15];
-    int e = 0;
-#pragma unroll
-    for (int a = 0; a < 6; ++a) {
-#pragma unroll
-      for (int b = a; b < 6; ++b) {
-        add_dot2(acc[e], cmp[e], ji[a], ji[b], ji[6 + a], ji[6 + b]);
-        ++e;
-      }
+    if constexpr (sizeof(T) == sizeof(float)) {
+      add_image_key<kAddFold>(acc, cmp, rec);
+    } else if (!chain && !whole) {
+      add_image_key<kAddChain>(acc, cmp, rec);
+      chain = true;
+    } else {
+      if (first)
+        add_image_key<kAddFirst>(acc, cmp, rec);
+      else
+        add_image_key<kAddFold>(acc, cmp, rec);
+      first = chain = false;
     }
-#pragma unroll
-    for (int a = 0; a < 6; ++a) add_dot2(acc[21 + a], cmp[21 + a], ji[a], r0, ji[6 + a], r1);
   }
+  int base, count;
   if constexpr (sizeof(T) == sizeof(float)) {
 #pragma unroll
     for (int e = 0; e < 27; ++e) acc[e] -= cmp[e];
+    warp_scatter_sums<27>(acc, lane, base, count);
+    if (count > 0) d.img_item_partial[kImageItemStride<T> * wid + base] = double(acc[0]);
+  } else {
+    if (whole || it.z - it.y != 64) {   // (two keys a lane, chained: all of it is in acc)
+#pragma unroll
+      for (int e = 0; e < 27; ++e) acc[e] += cmp[e];
+    }
+    warp_scatter_sums<27, 16, 2>(acc, lane, base, count);
+    // the last level: of the (up to) two values, one kept and one given
+    const bool up = (lane & 1) != 0;
+    const T keep = up ? acc[1] : acc[0], give = up ? acc[0] : acc[1];
+    T lo;
+    const T hi = two_sum(keep, __shfl_xor_sync(0xffffffffu, give, 1), lo);
+    if (up ? count == 2 : count > 0) {
+      double* out = d.img_item_partial + kImageItemStride<T> * wid + base + (up ? 1 : 0);
+      out[0] = hi;
+      out[28] = lo;
+    }
   }
-  int base, count;
-  warp_scatter_sums<27>(acc, lane, base, count);
-  if (count > 0) d.img_item_partial[28LL * wid + base] = double(acc[0]);
 }
 
 __global__ void __launch_bounds__(256) k_image_finalize(DevPlan d) {
@@ -1372,14 +1441,28 @@ __global__ void __launch_bounds__(256) k_image_finalize(DevPlan d) {
   if (lane < 27) {
     const double* part = d.img_item_partial + lane;
     if (d.precision == GBA_PRECISION_MIXED) {
-      for (int t = ib; t < ie; ++t) v += part[28LL * t];
-    } else {   // finer items (image_item_size): four interleaved sums
-      double s[4] = {0.0, 0.0, 0.0, 0.0};
-      for (int t = ib; t < ie; t += 4)
+      for (int t = ib; t < ie; ++t) v += part[kImageItemStride<float> * t];
+    } else {   // finer items (image_item_size): four interleaved compensated sums
+      double s[4], c[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const double* p = part + kImageItemStride<double> * (ib + u);
+        s[u] = ib + u < ie ? p[0] : 0.0;
+        c[u] = ib + u < ie ? p[28] : 0.0;
+      }
+      for (int t = ib + 4; t < ie; t += 4)
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-          if (t + u < ie) s[u] += part[28LL * (t + u)];
-      v = (s[0] + s[1]) + (s[2] + s[3]);
+          if (t + u < ie) {
+            const double* p = part + kImageItemStride<double> * (t + u);
+            const double y = p[0] + c[u], n = s[u] + y;
+            c[u] = (y - (n - s[u])) + p[28];
+            s[u] = n;
+          }
+      double e0, e1, e2;
+      const double a = two_sum(s[0], s[1], e0), b = two_sum(s[2], s[3], e1);
+      v = two_sum(a, b, e2);
+      v += ((c[0] + c[1]) + (c[2] + c[3])) + ((e0 + e1) + e2);
     }
   }
   // lane e holds entry e of (upper U in row order, then g)

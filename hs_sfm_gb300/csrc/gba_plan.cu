@@ -1470,7 +1470,8 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
   D.n_img_items = int(img_items.size());
   D.img_items = arena.upload(img_items);
   D.img_item_off = arena.upload(img_item_off);
-  D.img_item_partial = arena.alloc<double>(28 * std::max<size_t>(img_items.size(), 1));
+  D.img_item_partial = arena.alloc<double>((mixed ? kImageItemStride<float> : kImageItemStride<double>) *
+                                           std::max<size_t>(img_items.size(), 1));
   // with free cameras each parity has its own camera arrays (the fixed
   // cameras' values in both)
   D.cam64[0] = arena.upload(cam64);

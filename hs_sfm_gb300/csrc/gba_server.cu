@@ -277,7 +277,8 @@ int64_t gba_estimate_device_bytes(const gba_problem* p, int32_t precision) {
   if (precision == GBA_PRECISION_MIXED) b += K * 16 + P * 48 + I * 192;   // double-float mirrors
   b += P * (4 + 4 + 48 + 24 + 24 * tsz + 24);                 // offsets, x, x0, PV, PS, sums
   b += I * (4 * 4 + 48 + 96 + 48 + 192 + 24 * tsz + 288 + 48 + 6 * tsz + 28 * 8);
-  b += img_items * (16 + 28 * 8) + key_chunks * (16 + 16);    // image reduce items, key chunks and their sums
+  b += img_items * (16 + (mixed ? gba::kImageItemStride<float> : gba::kImageItemStride<double>) * 8);   // image reduce items
+  b += key_chunks * (16 + 16);                                // key chunks and their sums
   b += C * (80 + 40 + 80);
   b += n * n * tsz + nt * 1024 * tsz;                          // reduced system, tile inverses
   b += pairs * 8 + items * (16 + 352) + blocks * 12 + Ie * Ie * 4;
