@@ -3242,6 +3242,8 @@ __global__ void __launch_bounds__(kDfThreads, 1) k_chol_dataflow(DevPlan d) {
   const LMState& st = d.state[p];
   const bool run = st.active && !d.factor_flag[p];
   if (run) {
+    if (tr)   // (a launch with nothing to do keeps the last one's)
+      for (int e = tid; e < 4 * kDfTraceCap; e += blockDim.x) tr[e] = 0ull;
     for (int t = tid; t < nown; t += blockDim.x) {
       const int2 tl = d.df_own[ob + t];
       ti_s[t] = tl.x;
@@ -4748,8 +4750,6 @@ int run_cholesky_factor(const DevPlan& d, cudaStream_t s) {
     return 1;
   }
   if (d.df_grid > 0) {
-    if (d.df_trace)
-      cudaMemsetAsync(d.df_trace, 0, sizeof(unsigned long long) * 4 * kDfTraceCap * size_t(d.df_grid), s);
     DevPlan dd = d;
     void* args[] = {&dd};
     const cudaError_t e = cudaLaunchCooperativeKernel(

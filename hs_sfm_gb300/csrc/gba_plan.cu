@@ -1686,7 +1686,9 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
       const char* tp = std::getenv("GBA_FACTOR_TRACE");
       if (tp && *tp) {   // diagnostics: task timeline of the factorization, written at sync
         trace_path = tp;
-        D.df_trace = arena.alloc<unsigned long long>(size_t(grid) * kDfTraceCap * 4);
+        const size_t entries = size_t(grid) * kDfTraceCap * 4;
+        D.df_trace = arena.alloc<unsigned long long>(entries);
+        GBA_CUDA(cudaMemsetAsync(D.df_trace, 0, sizeof(unsigned long long) * entries, stream));
       }
     }
   }
@@ -2618,7 +2620,7 @@ int gba_solve_batch_into(const gba_problem* problems, const double* const* near_
   phase("x0 uploaded");
   if (!err) err = gba_plan_run(plan);
   phase("launched");
-  if (!err && (!plan->impl.passes_pending || plan->impl.h_pcg_extra))
+  if (!err && (!plan->impl.passes_pending || plan->impl.h_pcg_extra || plan->impl.d.df_trace))
     err = gba_plan_synchronize(plan);   // (else get_all waits and counts the loop's passes)
   phase("solved");
   if (!err) err = get_all(plan->impl, x_out, reports);
