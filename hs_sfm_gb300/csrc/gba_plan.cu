@@ -448,8 +448,11 @@ struct Plan {
   cudaStream_t side_stream = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   unsigned long long pcg_extra_seen = 0;
-  // the device-side iteration loop: the stream its body is captured on, and
-  // whether the last run's passes beyond the first are still to be counted
+  // the device-side iteration loop: whether the plan's runs iterate in it
+  // (decided once, when the plan is made: its graphs keep the choice), the
+  // stream its body is captured on, and whether the last run's passes beyond
+  // the first are still to be counted
+  bool loop = false;
   cudaStream_t loop_stream = nullptr;
   bool passes_pending = false;
   bool ran = false;
@@ -515,7 +518,6 @@ struct Plan {
   enum Part { kAll, kPrologue, kIteration, kEpilogue };
   void enqueue(bool profile, Part part = kAll, cudaStream_t on = nullptr,
                const cudaGraphConditionalHandle* loop = nullptr);
-  bool iterates_in_loop() const;
   void capture_loop();
   void count_passes(int passes);
   int run();
@@ -1838,6 +1840,15 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
   D.pt_chunk_sum = arena.alloc<double>(3 * std::max<size_t>(pt_chunks.size(), 1));
   D.img_chunk_sum = arena.alloc<double>(3 * std::max<size_t>(img_chunks.size(), 1));
   D.launch_counter = nullptr;
+  // The iterations are a device-side loop when a stopping test may end them
+  // early.  Unrolled, the launches after the last problem's stop find nothing
+  // to do but still take about 2 us each (a small FP64 problem of 8 iterations
+  // spent 1.3 ms of 2.8 in the other 42 of its 50).  A fixed number of
+  // iterations keeps the unrolled sequence, whose launches follow each other
+  // without the loop's turns.  GBA_UNROLLED=1 keeps it always, for comparison.
+  loop = !opt.profile && opt.max_iterations >= 4 &&
+         (opt.eps1 > 0.0 || opt.eps2 > 0.0 || opt.function_tolerance > 0.0) &&
+         std::getenv("GBA_UNROLLED") == nullptr;
   GBA_CUDA(cudaMemsetAsync(D.state, 0, sizeof(LMState) * nprob, stream));
   arena.flush();
   phase("uploads issued");
@@ -1856,18 +1867,6 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
     }
   }
   return GBA_OK;
-}
-
-// Whether a run's iterations are a device-side loop: when a stopping test
-// may end them early.  Unrolled, the launches after the last problem's stop
-// find nothing to do but still take about 2 us each (a small FP64 problem of
-// 8 iterations spent 1.3 ms of 2.8 in the other 42 of its 50).  A fixed number
-// of iterations keeps the unrolled sequence, whose launches follow each other
-// without the loop's turns.  GBA_UNROLLED=1 keeps it always, for comparison.
-bool Plan::iterates_in_loop() const {
-  return !opt.profile && opt.max_iterations >= 4 &&
-         (opt.eps1 > 0.0 || opt.eps2 > 0.0 || opt.function_tolerance > 0.0) &&
-         std::getenv("GBA_UNROLLED") == nullptr;
 }
 
 // Adds the iteration loop to the graph `stream` is being captured into: a
@@ -2026,7 +2025,6 @@ int Plan::run() {
   GBA_CUDA(cudaSetDevice(device));
   cudaGetLastError();   // a stale error from other code on this thread is not ours
   GBA_CUDA(cudaEventRecord(ev0, stream));
-  const bool loop = iterates_in_loop();
   passes_pending = loop;
   if (opt.use_cuda_graph) {
     if (!graph_exec) {
