@@ -77,6 +77,7 @@ struct LMState {
   int first;      // the first linearization (sets mu0)
   int pcg_iters;
   int loop_passes;  // problem 0: passes of the run's device-side iteration loop
+  long long loop_total;  // problem 0: the same of all runs of the plan
 };
 
 // Per-problem constant description (device).

@@ -683,6 +683,7 @@ __global__ void k_init(DevPlan d) {
     st.factor_ok = 1;
     st.stop = GBA_STOP_MAX_ITERATIONS;
     st.status = GBA_OK;
+    st.loop_total = d.state[p].loop_total;   // (of the plan, not of this run)
     d.state[p] = st;
     d.factor_flag[p] = 0;
   }
@@ -4549,6 +4550,7 @@ __global__ void __launch_bounds__(256) k_ctrl_loop(DevPlan d, cudaGraphCondition
   any = __syncthreads_or(any);
   if (threadIdx.x == 0) {
     const int passes = ++d.state[0].loop_passes;
+    ++d.state[0].loop_total;
     cudaGraphSetConditional(h, any && passes <= d.max_iterations ? 1u : 0u);
   }
 }

@@ -450,11 +450,12 @@ struct Plan {
   unsigned long long pcg_extra_seen = 0;
   // the device-side iteration loop: whether the plan's runs iterate in it
   // (decided once, when the plan is made: its graphs keep the choice), the
-  // stream its body is captured on, and whether the last run's passes beyond
-  // the first are still to be counted
+  // stream its body is captured on, the runs whose passes beyond the first are
+  // still to be counted, and the passes of all counted runs
   bool loop = false;
   cudaStream_t loop_stream = nullptr;
-  bool passes_pending = false;
+  int runs_uncounted = 0;
+  long long passes_seen = 0;
   bool ran = false;
   long long launches_last_run = 0;
   double setup_ms = 0;
@@ -519,7 +520,7 @@ struct Plan {
   void enqueue(bool profile, Part part = kAll, cudaStream_t on = nullptr,
                const cudaGraphConditionalHandle* loop = nullptr);
   void capture_loop();
-  void count_passes(int passes);
+  void count_passes(const LMState& st);
   int run();
   int sync();
 };
@@ -1901,13 +1902,14 @@ void Plan::capture_loop() {
   GBA_CUDA(cudaStreamUpdateCaptureDependencies(stream, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
 }
 
-// The loop ran `passes` passes in the last run; one is counted already.
-void Plan::count_passes(int passes) {
-  if (!passes_pending) return;
-  passes_pending = false;
-  const long long extra = iter_launches * (long long)(passes - 1);
-  launches_last_run += extra;
-  g_launches += extra;
+// Adds the launches of the loop's passes of the runs not yet counted (one pass
+// of each is counted already); st: problem 0's state after the last of them.
+void Plan::count_passes(const LMState& st) {
+  if (runs_uncounted == 0) return;
+  g_launches += iter_launches * (st.loop_total - passes_seen - runs_uncounted);
+  launches_last_run += iter_launches * (long long)(st.loop_passes - 1);
+  passes_seen = st.loop_total;
+  runs_uncounted = 0;
 }
 
 // The launch sequence of one solve.  When profiling, an event is recorded
@@ -2025,7 +2027,6 @@ int Plan::run() {
   GBA_CUDA(cudaSetDevice(device));
   cudaGetLastError();   // a stale error from other code on this thread is not ours
   GBA_CUDA(cudaEventRecord(ev0, stream));
-  passes_pending = loop;
   if (opt.use_cuda_graph) {
     if (!graph_exec) {
       cudaGraph_t g;
@@ -2092,6 +2093,7 @@ int Plan::run() {
   }
   GBA_CUDA(cudaEventRecord(ev1, stream));
   g_launches += launches_last_run;
+  if (loop) ++runs_uncounted;
   ran = true;
   return GBA_OK;
 }
@@ -2107,10 +2109,10 @@ int Plan::sync() {
     launches_last_run += extra;
     g_launches += extra;
   }
-  if (passes_pending) {
+  if (runs_uncounted > 0) {
     LMState st;
     GBA_CUDA(cudaMemcpy(&st, d.state, sizeof(st), cudaMemcpyDeviceToHost));
-    count_passes(st.loop_passes);
+    count_passes(st);
   }
   if (d.df_trace && !trace_path.empty()) write_trace();
   if (opt.profile) {
@@ -2408,7 +2410,7 @@ int get_all(gba::Plan& P, double* const* xs, gba_report* reports) {
     GBA_CUDA(cudaStreamSynchronize(P.stream));
     std::vector<gba::LMState> st(P.B);
     GBA_CUDA(cudaMemcpy(st.data(), P.d.state, sizeof(gba::LMState) * P.B, cudaMemcpyDeviceToHost));
-    P.count_passes(st[0].loop_passes);
+    P.count_passes(st[0]);
     const long long np = 3LL * P.d.P, ni = 6LL * P.d.I, nc = P.d.free_cams ? 10LL * P.d.Ctot : 0;
     const size_t nx = size_t(np + ni + nc);
     gba::HostBuf<double> stage(nx);
@@ -2519,7 +2521,7 @@ int gba_plan_last_run_launches(gba_plan* p, int64_t* n) {
   if (!p || !n) return GBA_ERR_INVALID;
   return guarded([&] {
     // the loop's passes are known once the run is over
-    if (p->impl.passes_pending && gba_plan_query(p) == GBA_OK)
+    if (p->impl.runs_uncounted > 0)
       if (int e = p->impl.sync()) return e;
     *n = p->impl.launches_last_run;
     return GBA_OK;
@@ -2618,7 +2620,7 @@ int gba_solve_batch_into(const gba_problem* problems, const double* const* near_
   phase("x0 uploaded");
   if (!err) err = gba_plan_run(plan);
   phase("launched");
-  if (!err && (!plan->impl.passes_pending || plan->impl.h_pcg_extra || plan->impl.d.df_trace))
+  if (!err && (!plan->impl.loop || plan->impl.h_pcg_extra || plan->impl.d.df_trace))
     err = gba_plan_synchronize(plan);   // (else get_all waits and counts the loop's passes)
   phase("solved");
   if (!err) err = get_all(plan->impl, x_out, reports);

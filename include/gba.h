@@ -328,7 +328,9 @@ GBA_API int gba_plan_get_report(gba_plan* plan, int32_t problem, gba_report* rep
 GBA_API int gba_plan_last_run_ms(gba_plan* plan, double* ms);
 GBA_API int gba_plan_kernel_stats(gba_plan* plan, int32_t stage, double* total_ms,
                           int32_t* launches);
-/* Counts of this library's kernel launches in the last run. */
+/* Counts of this library's kernel launches in the last run.  Waits for a run
+ * with stopping tests, whose iterations a device-side loop counts; until a
+ * call waits for such a run, gba_kernel_launch_count has one iteration of it. */
 GBA_API int gba_plan_last_run_launches(gba_plan* plan, int64_t* launches);
 /* Device bytes the plan holds (every buffer of its arena). */
 GBA_API int gba_plan_device_bytes(gba_plan* plan, int64_t* bytes);
