@@ -21,7 +21,7 @@
 //    length (tri_order), so that a warp's lanes have the same number of views
 //    (2 to 12 views: the longest of 32 is 12, the mean 7);
 //  - a batch that does not fill the schedulers' lanes twice runs 2, 4 or 8
-//    lanes per track, which share its views and add their sums by shuffles:
+//    lanes per track, which share its views and its sums' entries (RowSums):
 //    its time is one warp's instruction count;
 //  - the candidate's cost and normal equations are formed in one pass (nearly
 //    every step is accepted), and the eigenvector comes from inverse iteration
@@ -100,73 +100,126 @@ __device__ __forceinline__ void ld2(const double* __restrict__ p, double* o) {
   }
 }
 
-// The sums of a track's lanes: every lane of the group of G gets the same bits.
-template <int G, int N>
-__device__ __forceinline__ void group_sum(double* v, unsigned mask) {
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1)
-#pragma unroll
-    for (int e = 0; e < N; ++e) v[e] += __shfl_xor_sync(mask, v[e], o);
-}
+// The sums over a track's views of two rows' products, in the views' order
+// whatever G, so a track has the same bits in any batch.  Each view gives two
+// rows of four values; entry e of the sums is the e-th (r, c), r <= c, of the
+// 4 x 4 upper triangle: sum += ra[r] ra[c], then rb[r] rb[c].  A group's lanes
+// form the rows of G views at a time; its entries are shared out over the
+// lanes, which read the rows one after the other from shared memory: of the
+// FP64 pipe's instructions only 2 to 10 a view instead of 20.  (Sums added by
+// shuffles in a tree cost the same, 0.097 ms against 0.095 for 3,001 tracks,
+// but a track's last digits then changed with the size of its batch.)
+template <int G>
+struct RowSums {
+  static constexpr int kOwn = (10 + G - 1) / G;
+  double acc[kOwn];
+  double (*buf)[8];   // the group's rows [G][8] (G > 1)
+  int sub;
+  unsigned mask;
 
-// Cost, normal matrix and gradient of a track at X: s = (F, N00 N01 N02 N11
-// N12 N22, g0 g1 g2), this lane's views sub, sub + G, ... summed over the group.
+  __device__ __forceinline__ RowSums(double (*rows)[8], int sub_, unsigned mask_)
+      : buf(G > 1 ? rows + threadIdx.x / G * G : rows), sub(sub_), mask(mask_) {
+#pragma unroll
+    for (int u = 0; u < kOwn; ++u) acc[u] = 0.0;
+  }
+  static __device__ __forceinline__ int row(int e) { return e < 4 ? 0 : e < 7 ? 1 : e < 9 ? 2 : 3; }
+  static __device__ __forceinline__ int col(int e) { return e < 4 ? e : e < 7 ? e - 3 : e < 9 ? e - 5 : 3; }
+  // The rows of the next `views` (at most G) views, the sub-th of them this lane's.
+  __device__ __forceinline__ void add(const double ra[4], const double rb[4], int views) {
+    if constexpr (G == 1) {
+#pragma unroll
+      for (int e = 0; e < 10; ++e) acc[e] = fma(rb[row(e)], rb[col(e)], fma(ra[row(e)], ra[col(e)], acc[e]));
+    } else {
+      __syncwarp(mask);   // (the last rows are read)
+      if (sub < views) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          buf[sub][c] = ra[c];
+          buf[sub][4 + c] = rb[c];
+        }
+      }
+      __syncwarp(mask);
+      for (int l = 0; l < views; ++l) {
+#pragma unroll
+        for (int u = 0; u < kOwn; ++u) {
+          const int e = min(sub + G * u, 9);
+          const double* v = buf[l];
+          acc[u] = fma(v[4 + row(e)], v[4 + col(e)], fma(v[row(e)], v[col(e)], acc[u]));
+        }
+      }
+    }
+  }
+  // Every lane gets the ten sums.
+  __device__ __forceinline__ void get(double s[10]) {
+    if constexpr (G == 1) {
+#pragma unroll
+      for (int e = 0; e < 10; ++e) s[e] = acc[e];
+    } else {
+      double* all = buf[0];
+      __syncwarp(mask);
+#pragma unroll
+      for (int u = 0; u < kOwn; ++u)
+        if (sub + G * u < 10) all[sub + G * u] = acc[u];
+      __syncwarp(mask);
+#pragma unroll
+      for (int e = 0; e < 10; ++e) s[e] = all[e];
+    }
+  }
+};
+
+// Normal matrix, gradient and cost of a track at X: s = (N00 N01 N02 g0 N11
+// N12 g1 N22 g2 F), the upper triangle of the sums over (J, residual).
 template <int G>
 __device__ __forceinline__ void tri_normal(const double* __restrict__ views, const long long* __restrict__ tv,
                                            const double* __restrict__ keys, int m, int sub, unsigned mask,
-                                           const double X[3], double s[10]) {
+                                           double (*rows)[8], const double X[3], double s[10]) {
+  RowSums<G> sums(rows, sub, mask);
+  for (int base = 0; base < m; base += G) {
+    const int i = base + sub;
+    double J[2][4] = {};   // (d key / d X, residual) of u and v
+    if (i < m) {
+      double w[22];   // f s cx cy fa k1 k2 k3 d1 d2 R C
+      ld2<22>(views + kViewDoubles * tv[i], w);
+      const double* R = w + 10;
+      const double e0 = X[0] - w[19], e1 = X[1] - w[20], e2 = X[2] - w[21];
+      const double c0 = fma(R[2], e2, fma(R[1], e1, R[0] * e0));
+      const double c1 = fma(R[5], e2, fma(R[4], e1, R[3] * e0));
+      const double c2 = fma(R[8], e2, fma(R[7], e1, R[6] * e0));
+      const double iz = 1.0 / c2;
+      const double x = c0 * iz, y = c1 * iz;
+      const double r2 = fma(y, y, x * x);
+      const double k1 = w[5], k2 = w[6], k3 = w[7], d1 = w[8], d2 = w[9];
+      const double c = r2 * fma(r2, fma(r2, k3, k2), k1);
+      const double x2 = x + x, y2 = y + y, xy2 = x2 * y;
+      const double ex = fma(d1, xy2, fma(d2, fma(x2, x, r2), fma(c, x, x)));
+      const double ey = fma(d2, xy2, fma(d1, fma(y2, y, r2), fma(c, y, y)));
+      const double f = w[0], sk = w[1], fa = w[4];
+      J[0][3] = fma(f, ex, fma(sk, ey, w[2])) - keys[2 * i];
+      J[1][3] = fma(fa, ey, w[3]) - keys[2 * i + 1];
+      // d key / d (x, y), then by the camera point (b), then by X
+      const double dc = 2.0 * fma(r2, fma(r2, 3.0 * k3, 2.0 * k2), k1);
+      const double t = dc * x, q = 1.0 + c;
+      const double exx = fma(t, x, fma(d1, y2, fma(3.0 * d2, x2, q)));
+      const double exy = fma(t, y, fma(d1, x2, d2 * y2));
+      const double eyy = fma(dc * y, y, fma(d2, x2, fma(3.0 * d1, y2, q)));
+      const double bx[2] = {fma(f, exx, sk * exy) * iz, fa * exy * iz};
+      const double by[2] = {fma(f, exy, sk * eyy) * iz, fa * eyy * iz};
 #pragma unroll
-  for (int e = 0; e < 10; ++e) s[e] = 0.0;
-  for (int i = sub; i < m; i += G) {
-    double w[22];   // f s cx cy fa k1 k2 k3 d1 d2 R C
-    ld2<22>(views + kViewDoubles * tv[i], w);
-    const double* R = w + 10;
-    const double e0 = X[0] - w[19], e1 = X[1] - w[20], e2 = X[2] - w[21];
-    const double c0 = fma(R[2], e2, fma(R[1], e1, R[0] * e0));
-    const double c1 = fma(R[5], e2, fma(R[4], e1, R[3] * e0));
-    const double c2 = fma(R[8], e2, fma(R[7], e1, R[6] * e0));
-    const double iz = 1.0 / c2;
-    const double x = c0 * iz, y = c1 * iz;
-    const double r2 = fma(y, y, x * x);
-    const double k1 = w[5], k2 = w[6], k3 = w[7], d1 = w[8], d2 = w[9];
-    const double c = r2 * fma(r2, fma(r2, k3, k2), k1);
-    const double x2 = x + x, y2 = y + y, xy2 = x2 * y;
-    const double ex = fma(d1, xy2, fma(d2, fma(x2, x, r2), fma(c, x, x)));
-    const double ey = fma(d2, xy2, fma(d1, fma(y2, y, r2), fma(c, y, y)));
-    const double f = w[0], sk = w[1], fa = w[4];
-    const double u = fma(f, ex, fma(sk, ey, w[2])), v = fma(fa, ey, w[3]);
-    const double q0 = u - keys[2 * i], q1 = v - keys[2 * i + 1];
-    s[0] = fma(q1, q1, fma(q0, q0, s[0]));
-    // d key / d (x, y), then by the camera point (b), then by X
-    const double dc = 2.0 * fma(r2, fma(r2, 3.0 * k3, 2.0 * k2), k1);
-    const double t = dc * x, q = 1.0 + c;
-    const double exx = fma(t, x, fma(d1, y2, fma(3.0 * d2, x2, q)));
-    const double exy = fma(t, y, fma(d1, x2, d2 * y2));
-    const double eyy = fma(dc * y, y, fma(d2, x2, fma(3.0 * d1, y2, q)));
-    const double bx[2] = {fma(f, exx, sk * exy) * iz, fa * exy * iz};
-    const double by[2] = {fma(f, exy, sk * eyy) * iz, fa * eyy * iz};
-    double J[6];
+      for (int r = 0; r < 2; ++r) {
+        const double bz = -fma(bx[r], x, by[r] * y);
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const double bz = -fma(bx[r], x, by[r] * y);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) J[3 * r + j] = fma(bz, R[6 + j], fma(by[r], R[3 + j], bx[r] * R[j]));
+        for (int j = 0; j < 3; ++j) J[r][j] = fma(bz, R[6 + j], fma(by[r], R[3 + j], bx[r] * R[j]));
+      }
     }
-    s[1] = fma(J[3], J[3], fma(J[0], J[0], s[1]));
-    s[2] = fma(J[3], J[4], fma(J[0], J[1], s[2]));
-    s[3] = fma(J[3], J[5], fma(J[0], J[2], s[3]));
-    s[4] = fma(J[4], J[4], fma(J[1], J[1], s[4]));
-    s[5] = fma(J[4], J[5], fma(J[1], J[2], s[5]));
-    s[6] = fma(J[5], J[5], fma(J[2], J[2], s[6]));
-    s[7] = fma(J[3], q1, fma(J[0], q0, s[7]));
-    s[8] = fma(J[4], q1, fma(J[1], q0, s[8]));
-    s[9] = fma(J[5], q1, fma(J[2], q0, s[9]));
+    sums.add(J[0], J[1], min(G, m - base));
   }
-  group_sum<G, 10>(s, mask);
+  sums.get(s);
 }
 
-// (N + mu I) d = g by a 3x3 Cholesky; false when not positive definite.
-__device__ __forceinline__ bool tri_solve(const double* N, double mu, const double* g, double d[3]) {
+// (N + mu I) d = g (of tri_normal's sums) by a 3x3 Cholesky; false when not
+// positive definite.
+__device__ __forceinline__ bool tri_solve(const double s[10], double mu, double d[3]) {
+  const double N[6] = {s[0], s[1], s[2], s[4], s[5], s[7]}, g[3] = {s[3], s[6], s[8]};
   const double a00 = N[0] + mu, a11 = N[3] + mu, a22 = N[5] + mu;
   if (!(a00 > 0.0)) return false;
   const double i0 = rsqrt(a00), l10 = N[1] * i0, l20 = N[2] * i0;
@@ -308,6 +361,7 @@ __global__ void __launch_bounds__(128) k_triangulate(long long n, const int* __r
                                                      const double* __restrict__ track_keys,
                                                      const double* __restrict__ views, TriParams prm,
                                                      double* __restrict__ points, int* __restrict__ status) {
+  __shared__ double rows[G > 1 ? 128 : 1][8];
   const long long slot = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / G;
   if (slot >= n) return;
   const int sub = threadIdx.x % G;
@@ -323,44 +377,39 @@ __global__ void __launch_bounds__(128) k_triangulate(long long n, const int* __r
     st = GBA_ERR_INVALID;
   } else {
     // DLT normal matrix A^T A (upper triangle) of the undistorted keys
-    double M[10];
-#pragma unroll
-    for (int e = 0; e < 10; ++e) M[e] = 0.0;
-    for (int i = sub; i < m; i += G) {
-      const double* vw = views + kViewDoubles * tv[i];
-      double w[10], P[14];
-      ld2<10>(vw, w);
-      ld2<14>(vw + 22, P);   // P, 1 / f, 1 / (f a)
-      const double k1 = w[5], k2 = w[6], k3 = w[7], d1 = w[8], d2 = w[9];
-      const double y0 = (keys[2 * i + 1] - w[3]) * P[13];
-      const double x0 = (keys[2 * i] - w[2] - w[1] * y0) * P[12];
-      double x = x0, y = y0;
-      for (int it = 0; it < 5; ++it) {
-        const double r2 = fma(y, y, x * x);
-        const double rc = 1.0 / fma(r2, fma(r2, fma(r2, k3, k2), k1), 1.0);
-        const double x2 = x + x, xy2 = x2 * y;
-        const double dx = fma(d1, xy2, d2 * fma(x2, x, r2));
-        const double dy = fma(d2, xy2, d1 * fma(y + y, y, r2));
-        x = (x0 - dx) * rc;
-        y = (y0 - dy) * rc;
-      }
-      const double u = fma(w[0], x, fma(w[1], y, w[2])), v = fma(w[4], y, w[3]);
-      double a[4], b[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        a[c] = fma(u, P[8 + c], -P[c]);
-        b[c] = fma(v, P[8 + c], -P[4 + c]);
-      }
-      int e = 0;
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = r; c < 4; ++c) {
-          M[e] = fma(b[r], b[c], fma(a[r], a[c], M[e]));
-          ++e;
+    RowSums<G> sums(rows, sub, mask);
+    for (int base = 0; base < m; base += G) {
+      const int i = base + sub;
+      double a[4] = {}, b[4] = {};
+      if (i < m) {
+        const double* vw = views + kViewDoubles * tv[i];
+        double w[10], P[14];
+        ld2<10>(vw, w);
+        ld2<14>(vw + 22, P);   // P, 1 / f, 1 / (f a)
+        const double k1 = w[5], k2 = w[6], k3 = w[7], d1 = w[8], d2 = w[9];
+        const double y0 = (keys[2 * i + 1] - w[3]) * P[13];
+        const double x0 = fma(-w[1], y0, keys[2 * i] - w[2]) * P[12];
+        double x = x0, y = y0;
+        for (int it = 0; it < 5; ++it) {
+          const double r2 = fma(y, y, x * x);
+          const double rc = 1.0 / fma(r2, fma(r2, fma(r2, k3, k2), k1), 1.0);
+          const double x2 = x + x, xy2 = x2 * y;
+          const double dx = fma(d1, xy2, d2 * fma(x2, x, r2));
+          const double dy = fma(d2, xy2, d1 * fma(y + y, y, r2));
+          x = (x0 - dx) * rc;
+          y = (y0 - dy) * rc;
         }
+        const double u = fma(w[0], x, fma(w[1], y, w[2])), v = fma(w[4], y, w[3]);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          a[c] = fma(u, P[8 + c], -P[c]);
+          b[c] = fma(v, P[8 + c], -P[4 + c]);
+        }
+      }
+      sums.add(a, b, min(G, m - base));
     }
-    group_sum<G, 10>(M, mask);
+    double M[10];
+    sums.get(M);
     double h[4];
     tri_smallest_eigenvector(M, h);
     if (h[3] == 0.0) {
@@ -372,14 +421,15 @@ __global__ void __launch_bounds__(128) k_triangulate(long long n, const int* __r
       if (!(isfinite(X[0]) && isfinite(X[1]) && isfinite(X[2]))) st = GBA_ERR_NAN;
     }
     if (st == GBA_OK) {   // LM refinement
-      double s[10];   // F, N, g
-      tri_normal<G>(views, tv, keys, m, sub, mask, X, s);
-      bool found = fmax(fabs(s[7]), fmax(fabs(s[8]), fabs(s[9]))) <= prm.eps1;
-      double mu = prm.tau * fmax(s[1], fmax(s[4], s[6]));
+      double s[10];
+      tri_normal<G>(views, tv, keys, m, sub, mask, rows, X, s);
+      auto gradient = [&] { return fmax(fabs(s[3]), fmax(fabs(s[6]), fabs(s[8]))); };
+      bool found = gradient() <= prm.eps1;
+      double mu = prm.tau * fmax(s[0], fmax(s[4], s[7]));
       double nu = 2.0;
       for (int k = 0; !found && k < prm.max_iterations; ++k) {
         double d[3];
-        if (!tri_solve(s + 1, mu, s + 7, d)) {
+        if (!tri_solve(s, mu, d)) {
           mu *= nu;
           nu *= 2.0;
           continue;
@@ -389,15 +439,15 @@ __global__ void __launch_bounds__(128) k_triangulate(long long n, const int* __r
         if (sqrt(dn2) <= prm.eps2 * (xn + prm.eps2)) break;
         const double Xn[3] = {X[0] - d[0], X[1] - d[1], X[2] - d[2]};
         double sn[10];
-        tri_normal<G>(views, tv, keys, m, sub, mask, Xn, sn);
-        const double denom = fma(mu, dn2, fma(s[9], d[2], fma(s[8], d[1], s[7] * d[0])));
-        const double rho = (s[0] - sn[0]) / denom;
-        if (isfinite(sn[0]) && rho > 0.0) {
+        tri_normal<G>(views, tv, keys, m, sub, mask, rows, Xn, sn);
+        const double denom = fma(mu, dn2, fma(s[8], d[2], fma(s[6], d[1], s[3] * d[0])));
+        const double rho = (s[9] - sn[9]) / denom;
+        if (isfinite(sn[9]) && rho > 0.0) {
 #pragma unroll
           for (int e = 0; e < 3; ++e) X[e] = Xn[e];
 #pragma unroll
           for (int e = 0; e < 10; ++e) s[e] = sn[e];
-          found = fmax(fabs(s[7]), fmax(fabs(s[8]), fabs(s[9]))) <= prm.eps1;
+          found = gradient() <= prm.eps1;
           const double tt = 2.0 * rho - 1.0;
           mu *= fmax(1.0 / 3.0, 1.0 - tt * tt * tt);
           nu = 2.0;
@@ -406,7 +456,7 @@ __global__ void __launch_bounds__(128) k_triangulate(long long n, const int* __r
           nu *= 2.0;
         }
       }
-      if (!isfinite(s[0])) st = GBA_ERR_NAN;
+      if (!isfinite(s[9])) st = GBA_ERR_NAN;
     }
   }
   if (sub < 3) points[3 * j + sub] = sub == 0 ? X[0] : sub == 1 ? X[1] : X[2];
