@@ -296,8 +296,12 @@ __device__ __noinline__ void tri_jacobi(double A[16], double out[4]) {
 // The same by inverse iteration on A = L D L^T (Golub & Van Loan 8.2.2): A is
 // a sum of squares, so the unpivoted factorization is stable, and the
 // error falls by (smallest / next eigenvalue) a step.  M: the upper triangle,
-// rows.  Rank below three (no unique vector), no positive pivots, or no
-// settling in 16 steps (the two smallest eigenvalues close): Jacobi.
+// rows.  Rank below three (no unique vector), no positive pivots, no settling
+// in 16 steps (the two smallest eigenvalues close), or an eigenvalue below the
+// one found: Jacobi.  The last is a vector without a homogeneous coordinate (a
+// point at infinity), of which the start has no part.  It is ruled out when
+// the leading 3 x 3 block has no eigenvalue at or below the one found: the
+// second smallest of A is not below that block's smallest.
 __device__ __forceinline__ void tri_smallest_eigenvector(const double M[10], double x[4]) {
   const double trace = M[0] + M[4] + M[7] + M[9];
   const double tiny = 1e-13 * trace;
@@ -340,6 +344,12 @@ __device__ __forceinline__ void tri_smallest_eigenvector(const double M[10], dou
       }
       settled = diff <= 1e-29;
     }
+    // the block less the eigenvalue r is positive definite: its leading minors
+    // (m3: the determinant times a00)
+    const double l = r * (1.0 + 1e-9), a00 = M[0] - l, a11 = M[4] - l, a22 = M[7] - l;
+    const double m2 = fma(-M[1], M[1], a00 * a11), c12 = fma(a00, M[5], -(M[1] * M[2]));
+    const double m3 = fma(-c12, c12, m2 * fma(-M[2], M[2], a00 * a22));
+    settled = settled && a00 > 0.0 && m2 > 0.0 && m3 > 0.0;
   }
   if (!settled) {
     double A[16] = {M[0], M[1], M[2], M[3], M[1], M[4], M[5], M[6],
