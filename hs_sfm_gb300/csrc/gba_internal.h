@@ -41,8 +41,9 @@ constexpr long long kImageItemStride = sizeof(T) == sizeof(float) ? 28 : 56;   /
 // sizes: the grouping of its FP32 sums is part of its results.  The FP64 path
 // is bound by its FP64 pipe (64 cycles an instruction and warp), so a small
 // problem is cut finer, until its items, image lists and key chunks fill the
-// 608 warp schedulers; its sizes depend on the problem alone, so its bits
-// are the same in any batch.  Below 64 (two entries a lane) an item's own
+// 608 warp schedulers of the whole chip; its sizes depend on the problem
+// alone (not on the SMs a partition has), so its bits are the same in any batch
+// and on any part of the chip.  Below 64 (two entries a lane) an item's own
 // reduction outweighs its sums.
 inline int auto_item(long long count, long long pieces, int unit, int lo, int hi) {
   const long long per = (count + pieces * unit - 1) / (pieces * unit) * unit;

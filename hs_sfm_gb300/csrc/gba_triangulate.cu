@@ -579,10 +579,12 @@ extern "C" int gba_triangulate(const gba_triangulation* p, const gba_options* o,
       TRI_CUDA(cudaEventCreate(&ev[1]));
       TRI_CUDA(cudaEventRecord(ev[0], s));
     }
-    // lanes per track: while the batch leaves lanes of the schedulers (608
-    // warps) idle twice over; one thread per track above, ordered by length
-    // (n <= INT32_MAX: the order's indices)
-    const long long lanes = 2LL * 608 * 32;
+    // lanes per track: while the batch leaves lanes of the schedulers (four
+    // warps an SM) idle twice over; one thread per track above, ordered by
+    // length (n <= INT32_MAX: the order's indices)
+    int sms = 0;
+    TRI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, o->device));
+    const long long lanes = 2LL * 4 * sms * 32;
     const int G = n * 8 <= lanes ? 8 : n * 4 <= lanes ? 4 : n * 2 <= lanes ? 2 : 1;
     int* d_order = nullptr;
     if (G == 1 && n <= INT32_MAX) {
