@@ -281,7 +281,14 @@ int64_t gba_estimate_device_bytes(const gba_problem* p, int32_t precision) {
   b += key_chunks * (16 + 16);                                // key chunks and their sums
   b += C * (80 + 40 + 80);
   b += n * n * tsz + nt * 1024 * tsz;                          // reduced system, tile inverses
-  b += pairs * 8 + items * (16 + 352) + blocks * 12 + Ie * Ie * 4;
+  b += items * (16 + 352) + blocks * 12;
+  if (free_cams) {
+    b += pairs * 8 + Ie * Ie * 4;
+  } else {   // counted, placed and sorted on the device: keys and pairs twice, tables per image pair
+    long long hist = 0, scratch = 0;
+    gba::pairs_sort_scratch(pairs, int(P), &hist, &scratch);
+    b += pairs * 24 + (hist + scratch + gba::scan_scratch_ints(Ie * Ie)) * 4 + Ie * Ie * 12 + blocks * 8 + P * 8;
+  }
   if (free_cams) {
     b += recs * (20 * tsz + 12) + P * 4;                        // camera Z records, offsets
     b += K * 40 * tsz + img_items * 128 * 8 + I * (60 * 8 + 128 * 8 + 4);   // J_c (x2), sums, E, ext
