@@ -59,6 +59,20 @@ inline int key_item_size(int option, bool mixed, long long keys) {
   return option > 0 ? option : mixed ? kKeyChunk : auto_item(keys, 304, 128, 128, kKeyChunk);
 }
 
+// A plan's device memory: buffers below kArenaOwn share chunks, uploads up to
+// kArenaUpload blocks of kArenaChunk bytes too, every buffer aligned.
+constexpr size_t kArenaAlign = 256, kArenaOwn = size_t(256) << 10, kArenaChunk = size_t(1) << 20;
+constexpr size_t kArenaUpload = size_t(64) << 10;
+// What a plan holds beside the `asked` bytes of its buffers, at most: a chunk
+// and a block begun, the ends of the others (a chunk is left with less than
+// kArenaOwn free, a block with less than kArenaUpload), the alignment of some
+// 150 buffers.  At most 100 buffers are below kArenaOwn.
+inline long long arena_overhead(long long asked) {
+  const long long small = asked < 100LL * (long long)kArenaOwn ? asked : 100LL * (long long)kArenaOwn;
+  return 2LL * (long long)kArenaChunk + small * (long long)kArenaOwn / (long long)(kArenaChunk - kArenaOwn) +
+         150LL * (long long)kArenaAlign;
+}
+
 // Per-problem LM state (device).  Written only by the control kernels.
 struct LMState {
   double mu, nu;

@@ -317,11 +317,11 @@ class HostBuf {
 // flush() comes before any launch that reads an upload; the blocks' host side
 // is kept until drop_staging(), after the stream has been waited for.
 struct DeviceArena {
-  static constexpr size_t kAlign = 256, kOwn = size_t(256) << 10, kChunk = size_t(1) << 20;
-  static constexpr size_t kSmallUpload = size_t(64) << 10, kBlock = size_t(1) << 20;
+  static constexpr size_t kAlign = kArenaAlign, kOwn = kArenaOwn, kChunk = kArenaChunk;
+  static constexpr size_t kSmallUpload = kArenaUpload, kBlock = kArenaChunk;
   std::vector<void*> ptrs;
   cudaStream_t stream = nullptr;
-  size_t bytes = 0;
+  size_t bytes = 0;                  // taken from the device's pool
   long long uploaded = 0;
   char* chunk = nullptr;
   size_t chunk_left = 0;
@@ -333,6 +333,7 @@ struct DeviceArena {
     void* p = nullptr;
     GBA_CUDA(cudaMallocAsync(&p, n, stream));
     ptrs.push_back(p);
+    bytes += n;
     return static_cast<char*>(p);
   }
   char* raw(size_t n) {
@@ -350,7 +351,6 @@ struct DeviceArena {
   template <typename T>
   T* alloc(size_t count) {
     if (count == 0) count = 1;
-    bytes += count * sizeof(T);
     return reinterpret_cast<T*>(raw(count * sizeof(T)));
   }
   template <typename T>
@@ -368,7 +368,6 @@ struct DeviceArena {
       block = own(kBlock);
       used = sent = 0;
     }
-    bytes += size;
     std::memcpy(stages.back()->data() + used, h, size);
     T* p = reinterpret_cast<T*>(block + used);
     used += room;

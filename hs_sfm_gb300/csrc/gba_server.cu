@@ -296,7 +296,8 @@ int64_t gba_estimate_device_bytes(const gba_problem* p, int32_t precision) {
   }
   const int64_t rows = gba_y_size(p) - 2 * K;                   // constraint and prior rows
   if (rows > 0) b += rows * 32 + (P + I + 2) * 8 + p->number_of_point_priors * 96;
-  return b + (1 << 20);                                        // bookkeeping slack
+  b += 1 << 20;                                                // bookkeeping slack
+  return b + gba::arena_overhead(b);
 }
 
 void gba_default_server_config(gba_server_config* c) {

@@ -332,7 +332,8 @@ GBA_API int gba_plan_kernel_stats(gba_plan* plan, int32_t stage, double* total_m
  * with stopping tests, whose iterations a device-side loop counts; until a
  * call waits for such a run, gba_kernel_launch_count has one iteration of it. */
 GBA_API int gba_plan_last_run_launches(gba_plan* plan, int64_t* launches);
-/* Device bytes the plan holds (every buffer of its arena). */
+/* Device bytes the plan holds: what it has taken from the device's memory
+ * pool for its buffers. */
 GBA_API int gba_plan_device_bytes(gba_plan* plan, int64_t* bytes);
 /* Sizes of a plan's work lists (no counterpart in the reference: the
  * structure the device builds once per plan), for cost models and
@@ -442,8 +443,8 @@ GBA_API int gba_server_wait(gba_server* server, int64_t ticket, double timeout_m
  * discarded.  Later polls return GBA_ERR_CANCELLED. */
 GBA_API int gba_server_cancel(gba_server* server, int64_t ticket);
 GBA_API int gba_server_get_stats(gba_server* server, gba_server_stats* stats);
-/* Device bytes a plan for this problem would hold (host-side estimate used
- * for admission). */
+/* Device bytes a plan for this problem would hold at most (host-side estimate
+ * used for admission). */
 GBA_API int64_t gba_estimate_device_bytes(const gba_problem* problem, int32_t precision);
 
 /* ---- allocation-free cost ------------------------------------------------
