@@ -2682,27 +2682,35 @@ int gba_autotune(const gba_problem* problems, const double* const* near_ys, cons
     *ms_per_it = best / base.max_iterations;
     return GBA_OK;
   };
+  // the baseline: the sizes of option 0, by name in mixed precision (fixed
+  // sizes), 0 in FP64 (cut by the problem, and kept as 0)
+  const bool mixed = base.precision == GBA_PRECISION_MIXED;
+  const int default_pair = mixed ? gba::kPairItem : 0, default_image = mixed ? gba::kImageItem : 0,
+            default_key = mixed ? gba::kKeyChunk : 0;
+  int best_pair = default_pair, best_image = default_image, best_key = default_key;
   double t_default = 0.0;
-  if (int e = time_one(gba::kPairItem, gba::kImageItem, gba::kKeyChunk, &t_default, base.z_layout)) return e;
-  int best_pair = gba::kPairItem, best_image = gba::kImageItem, best_key = gba::kKeyChunk;
+  if (int e = time_one(best_pair, best_image, best_key, &t_default, base.z_layout)) return e;
   int best_layout = resolved_layout;
   double t_best = t_default;
-  for (int pi : {256, 512, 2048, 4096}) {
+  for (int pi : {256, 512, 1024, 2048, 4096}) {
     double t = 0.0;
-    if (time_one(pi, gba::kImageItem, gba::kKeyChunk, &t, best_layout) == GBA_OK && t < t_best) {
+    if (pi == default_pair) continue;
+    if (time_one(pi, best_image, best_key, &t, best_layout) == GBA_OK && t < t_best) {
       t_best = t;
       best_pair = pi;
     }
   }
-  for (int ii : {256, 1024}) {
+  for (int ii : {256, 512, 1024}) {
     double t = 0.0;
-    if (time_one(best_pair, ii, gba::kKeyChunk, &t, best_layout) == GBA_OK && t < t_best) {
+    if (ii == default_image) continue;
+    if (time_one(best_pair, ii, best_key, &t, best_layout) == GBA_OK && t < t_best) {
       t_best = t;
       best_image = ii;
     }
   }
-  for (int ki : {256, 512, 2048}) {
+  for (int ki : {256, 512, 1024, 2048}) {
     double t = 0.0;
+    if (ki == default_key) continue;
     if (time_one(best_pair, best_image, ki, &t, best_layout) == GBA_OK && t < t_best) {
       t_best = t;
       best_key = ki;

@@ -209,8 +209,10 @@ typedef struct gba_options {
  * default image_item and key_item, then image_item over {256, 512, 1024}
  * with the best pair_item, then key_item over {256, 512, 1024, 2048} with
  * the best two, then (options->z_layout auto) the other Z layout with the
- * best sizes.  out receives the fastest sizes and layout and their time per
- * LM iteration beside that of the defaults.  A status code. */
+ * best sizes.  In FP64 the sizes start from option 0 (cut by the problem), and
+ * a size for which no candidate is faster is returned as 0.  out receives the
+ * fastest sizes and layout and their time per LM iteration beside that of the
+ * defaults.  A status code. */
 typedef struct gba_tuning {
   int32_t pair_item;
   int32_t image_item;
