@@ -37,6 +37,7 @@
 //                     normal_equation_solver.hpp:270-392,422-443)
 //   PCG:             k_assemble_blocks, k_pcg_* (block-Jacobi PCG on the
 //                    explicit 6x6 blocks of S)
+#include "gba_factor_layout.h"
 #include "gba_internal.h"
 
 #include <cooperative_groups.h>
@@ -2737,15 +2738,6 @@ constexpr int kDfThreads = 256;
 template <typename T>
 __host__ __device__ constexpr int df_batch() { return 2; }
 
-// Tiles of row i kept by its own CTA: (i, i), (i, i-1) and, in FP32, (i, i-2).
-// An FP64 update takes 8 us of one SM's FP64 pipe, so a third tile would make
-// the row's updates slower than the chain they have to keep ahead of.
-template <typename T>
-__host__ __device__ constexpr int df_row_tiles() { return sizeof(T) == 4 ? 3 : 2; }
-// Tiles kept by row i's second CTA, left of those.
-template <typename T>
-__host__ __device__ constexpr int df_helper_tiles() { return sizeof(T) == 4 ? 3 : 0; }
-
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -5007,50 +4999,10 @@ bool dataflow_layout_t(int nt, int device, int* grid, int* max_own, int* rows, i
     return false;
   }
   if (!coop || nt < 2) return false;
-  const long long ntiles = (long long)nt * (nt + 1) / 2;
-  const int G = int(std::min<long long>(sms, ntiles));
-  // row i's last tiles go to CTA i mod G; the rest, heaviest first, to the
-  // CTA with the least work so far.  When there are at least twice as many
-  // CTAs as tile rows, the rows' CTAs take none of the rest (and run the
-  // rows' fixed program): a CTA busy with an update when its row's chain
-  // task becomes ready would delay the chain by that update
-  std::vector<std::vector<int2>> lists(G);
-  const bool dedicated = G >= 2 * nt;
-  const int row_tiles = dedicated ? df_row_tiles<T>() : 2;
-  const int helper_tiles = G >= 4 * nt ? df_helper_tiles<T>() : 0;
-  const int band = row_tiles + helper_tiles;   // tiles of a row kept by its own CTAs
-  *rows = dedicated ? nt : 0;
-  *helpers = helper_tiles > 0 ? nt : 0;
-  const int first_worker = *rows + *helpers;
-  std::vector<long long> load(G, 0);
-  for (int i = 0; i < nt; ++i) {
-    const int g = i % G;
-    for (int u = 0; u < row_tiles && u <= i; ++u) {
-      lists[g].push_back(make_int2(i, i - u));
-      load[g] += i - u + 1;
-    }
-    for (int u = row_tiles; u < band && u <= i; ++u) lists[nt + i].push_back(make_int2(i, i - u));
-  }
-  std::vector<int2> rest;
-  for (int j = 0; j < nt; ++j)
-    for (int i = j + band; i < nt; ++i) rest.push_back(make_int2(i, j));
-  std::stable_sort(rest.begin(), rest.end(), [](const int2& a, const int2& b) { return a.y > b.y; });
-  for (const int2& t : rest) {
-    int g = first_worker;
-    for (int h = first_worker + 1; h < G; ++h)
-      if (load[h] < load[g]) g = h;
-    lists[g].push_back(t);
-    load[g] += t.y + 1;
-  }
-  int mo = 0;
-  for (auto& l : lists) {
-    std::sort(l.begin(), l.end(), [](const int2& a, const int2& b) {
-      return a.y != b.y ? a.y < b.y : a.x < b.x;
-    });
-    mo = std::max(mo, int(l.size()));
-  }
+  const DfLayout l = df_layout(nt, sizeof(T) == sizeof(float), sms);
+  const int G = l.grid, mo = l.max_own;
   const size_t smem = df_smem_bytes<T>(mo);
-  if (mo > (dedicated ? 64 : kDfThreads) ||
+  if (mo > (l.rows > 0 ? kDfWorkerTiles : kDfThreads) ||
       !allow_dynamic_smem(reinterpret_cast<const void*>(&k_chol_dataflow<T>), smem))
     return false;
   int per_sm = 0;
@@ -5061,12 +5013,14 @@ bool dataflow_layout_t(int nt, int device, int* grid, int* max_own, int* rows, i
   }
   own_off->assign(1, 0);
   own->clear();
-  for (auto& l : lists) {
-    own->insert(own->end(), l.begin(), l.end());
+  for (const auto& o : l.own) {
+    for (const DfTile& t : o) own->push_back(make_int2(t.i, t.j));
     own_off->push_back(int(own->size()));
   }
   *grid = G;
   *max_own = mo;
+  *rows = l.rows;
+  *helpers = l.helpers;
   return true;
 }
 
