@@ -92,7 +92,7 @@ struct LMState {
   int first;      // the first linearization (sets mu0)
   int pcg_iters;
   int loop_passes;  // problem 0: passes of the run's device-side iteration loop
-  long long loop_total;  // problem 0: the same of all runs of the plan
+  long long loop_total;   // problem 0: the same of all runs of the plan
 };
 
 // Per-problem constant description (device).
@@ -325,9 +325,14 @@ int launch_ctrl_initial_cost(const DevPlan& d, cudaStream_t s);
 // accepted candidate's cost)
 int launch_linearize(const DevPlan& d, cudaStream_t s, bool keys = true);
 int launch_image_reduce(const DevPlan& d, cudaStream_t s);
-// loop (or null): the while node whose body this launch is in; it is told
-// whether any problem still iterates
-int launch_ctrl_after_linearize(const DevPlan& d, cudaStream_t s, const cudaGraphConditionalHandle* loop = nullptr);
+// The condition of the iteration loop's while node, and the most passes after
+// which it may still go on.
+struct LoopControl {
+  cudaGraphConditionalHandle handle;
+  int limit;
+};
+// loop (or null): the condition it sets
+int launch_ctrl_after_linearize(const DevPlan& d, cudaStream_t s, const LoopControl* loop = nullptr);
 int launch_point_schur(const DevPlan& d, cudaStream_t s);
 // plan build with Z planes: key_slot [K] = the inverse of img_keys, and the
 // assembly's pairs rewritten as slots

@@ -4531,19 +4531,18 @@ __global__ void k_ctrl_after_linearize(DevPlan d) {
   if (p < d.B) ctrl_after_linearize(d, p);
 }
 
-// The same in one CTA, inside the body of the iteration loop (a CUDA-graph
-// while node): the loop goes on while any problem does.  The pass in which the
-// last problem stops finds nothing to do in its other stages.  (Every pass of
-// an active problem counts an iteration; the bound on the passes only makes
-// the loop's end explicit.)
-__global__ void __launch_bounds__(256) k_ctrl_loop(DevPlan d, cudaGraphConditionalHandle h) {
+// The same in one CTA, in the body of the iteration loop (a CUDA-graph while
+// node): the loop goes on while any problem does and passes are left.  (Every
+// iteration of an active problem counts one, so where the control is at the
+// end of the body the limit only makes the loop's end explicit.)
+__global__ void __launch_bounds__(256) k_ctrl_loop(DevPlan d, LoopControl c) {
   int any = 0;
   for (int p = threadIdx.x; p < d.B; p += blockDim.x) any |= ctrl_after_linearize(d, p);
   any = __syncthreads_or(any);
   if (threadIdx.x == 0) {
     const int passes = ++d.state[0].loop_passes;
     ++d.state[0].loop_total;
-    cudaGraphSetConditional(h, any && passes <= d.max_iterations ? 1u : 0u);
+    cudaGraphSetConditional(c.handle, any && passes <= c.limit ? 1u : 0u);
   }
 }
 
@@ -4868,7 +4867,7 @@ int launch_image_reduce(const DevPlan& d, cudaStream_t s) {
   return 5;
 }
 
-int launch_ctrl_after_linearize(const DevPlan& d, cudaStream_t s, const cudaGraphConditionalHandle* loop) {
+int launch_ctrl_after_linearize(const DevPlan& d, cudaStream_t s, const LoopControl* loop) {
   if (loop) {
     k_ctrl_loop<<<1, 256, 0, s>>>(d, *loop);
     return 1;

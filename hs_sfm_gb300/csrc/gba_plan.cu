@@ -450,11 +450,11 @@ struct Plan {
   // the device-side iteration loop: whether the plan's runs iterate in it
   // (decided once, when the plan is made: its graphs keep the choice), the
   // stream its body is captured on, the runs whose passes beyond the first are
-  // still to be counted, and the passes of all counted runs
+  // still to be counted, the passes of all counted runs and a pass's launches
   bool loop = false;
   cudaStream_t loop_stream = nullptr;
   int runs_uncounted = 0;
-  long long passes_seen = 0;
+  long long passes_seen = 0, pass_launches = 0;
   bool ran = false;
   long long launches_last_run = 0;
   double setup_ms = 0;
@@ -515,9 +515,10 @@ struct Plan {
   // kIteration starts with the previous linearization's image sums and
   // control (beside the point Schur and the assembly, which do not need
   // them); kEpilogue runs them for the last iteration
-  enum Part { kAll, kPrologue, kIteration, kEpilogue };
-  void enqueue(bool profile, Part part = kAll, cudaStream_t on = nullptr,
-               const cudaGraphConditionalHandle* loop = nullptr);
+  // kBody is an iteration whose predecessor's sums and control are done, with
+  // its own at its end.  loop: the control's condition (or null)
+  enum Part { kAll, kPrologue, kIteration, kEpilogue, kBody };
+  void enqueue(bool profile, Part part = kAll, cudaStream_t on = nullptr, const LoopControl* loop = nullptr);
   void capture_loop();
   void count_passes(const LMState& st);
   int run();
@@ -1840,13 +1841,15 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
   D.pt_chunk_sum = arena.alloc<double>(3 * std::max<size_t>(pt_chunks.size(), 1));
   D.img_chunk_sum = arena.alloc<double>(3 * std::max<size_t>(img_chunks.size(), 1));
   D.launch_counter = nullptr;
-  // The iterations are a device-side loop when a stopping test may end them
-  // early.  Unrolled, the launches after the last problem's stop find nothing
-  // to do but still take about 2 us each (a small FP64 problem of 8 iterations
-  // spent 1.3 ms of 2.8 in the other 42 of its 50).  A fixed number of
-  // iterations keeps the unrolled sequence, whose launches follow each other
-  // without the loop's turns.  GBA_UNROLLED=1 keeps it always, for comparison.
-  loop = !opt.profile && opt.max_iterations >= 4 &&
+  // With a stopping test the iterations may end early, and are a device-side
+  // loop (capture_loop) from so many allowed on that skipping the rest pays: a
+  // resident plan's plain graph saves its turns (7 of 14 iterations 1.06-1.09
+  // ms in the loop, 1.14 plain, but 11 of 14 2.79 against 2.74 and all 14 1.95
+  // against 1.88; 7 of 10 1.09 against 1.07), a one-shot solve's replays cost
+  // as much as the turns (7 of 10 1.10 against 1.13 ms).  A fixed number of
+  // iterations keeps the plain sequence.  GBA_UNROLLED=1 keeps it always, for
+  // comparison.
+  loop = !opt.profile && opt.max_iterations >= (opt.use_cuda_graph ? 16 : 10) &&
          (opt.eps1 > 0.0 || opt.eps2 > 0.0 || opt.function_tolerance > 0.0) &&
          std::getenv("GBA_UNROLLED") == nullptr;
   GBA_CUDA(cudaMemsetAsync(D.state, 0, sizeof(LMState) * nprob, stream));
@@ -1869,10 +1872,26 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
   return GBA_OK;
 }
 
-// Adds the iteration loop to the graph `stream` is being captured into: a
-// while node whose body is one iteration (with the previous linearization's
-// sums and checks first, which also serve as the epilogue).
+// Adds the iterations of a run with stopping tests to the graph `stream` is
+// being captured into: a while node whose body is `iterations` LM iterations.
+// The body's control tells the node whether any problem goes on: it is the
+// check of the last linearization at the body's end, so the pass in which the
+// last problem stops is the last; a forked iteration starts with that check
+// (beside its Schur products), so there a stop is followed by an idle pass and
+// only the limit is known a pass ahead.
+//
+// An iteration after the last stop takes 13 to 16 us (its launches find nothing
+// to do), a turn of the node 3 to 7.  With one iteration to a turn a run that
+// used up its iterations took up to 8% longer than unrolled (22 images, mixed,
+// 50 iterations 4.06 ms against 3.75).  A resident plan takes four or five to a
+// turn, whichever leaves fewer over (3.81 ms; 10 images, FP64, 50 iterations
+// 6.13 against 6.05, but 7 of them 1.09 against 1.75); a forked iteration is
+// long enough for two (200 cameras, 20 iterations 9.67 against 9.60 ms, with
+// one 9.74); a one-shot solve, whose body is captured for its one run, takes
+// two (3.96 ms against 3.94 replayed from the host, 7 of 50 1.10 against 1.95).
 void Plan::capture_loop() {
+  const int limit = opt.max_iterations;
+  const int iterations = !opt.use_cuda_graph || side_stream ? 2 : (limit + 3) / 4 * 4 - limit <= (limit + 4) / 5 * 5 - limit ? 4 : 5;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   cudaGraph_t g = nullptr;
   const cudaGraphNode_t* deps = nullptr;
@@ -1890,34 +1909,48 @@ void Plan::capture_loop() {
   if (!loop_stream) GBA_CUDA(cudaStreamCreateWithFlags(&loop_stream, cudaStreamNonBlocking));
   GBA_CUDA(cudaStreamBeginCaptureToGraph(loop_stream, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                          cudaStreamCaptureModeThreadLocal));
+  const int passes = (limit + iterations - 1) / iterations;
+  const LoopControl control{h, side_stream ? passes - 1 : passes};
+  const int at = side_stream ? 0 : iterations - 1;   // the iteration with the control
   cudaGraph_t body = nullptr;
+  long long n = 0;
   try {
-    enqueue(false, kIteration, loop_stream, &h);
+    for (int it = 0; it < iterations; ++it) {
+      enqueue(false, side_stream ? kIteration : kBody, loop_stream, it == at ? &control : nullptr);
+      n += launches_last_run;
+    }
   } catch (...) {
     cudaStreamEndCapture(loop_stream, &body);
     throw;
   }
   GBA_CUDA(cudaStreamEndCapture(loop_stream, &body));
   GBA_CUDA(cudaStreamUpdateCaptureDependencies(stream, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
+  pass_launches = n;
+  if (side_stream) {   // (the last linearization's sums)
+    enqueue(false, kEpilogue);
+    n += launches_last_run;
+  }
+  launches_last_run = n;
 }
 
 // Adds the launches of the loop's passes of the runs not yet counted (one pass
 // of each is counted already); st: problem 0's state after the last of them.
 void Plan::count_passes(const LMState& st) {
   if (runs_uncounted == 0) return;
-  g_launches += iter_launches * (st.loop_total - passes_seen - runs_uncounted);
-  launches_last_run += iter_launches * (long long)(st.loop_passes - 1);
+  g_launches += pass_launches * (st.loop_total - passes_seen - runs_uncounted);
+  launches_last_run += pass_launches * (st.loop_passes - 1);
   passes_seen = st.loop_total;
   runs_uncounted = 0;
 }
 
 // The launch sequence of one solve.  When profiling, an event is recorded
 // after each stage and tagged with it.
-void Plan::enqueue(bool profile, Part part, cudaStream_t on, const cudaGraphConditionalHandle* loop) {
+void Plan::enqueue(bool profile, Part part, cudaStream_t on, const LoopControl* loop) {
   cudaStream_t s = on ? on : stream;
+  const bool nested = on != nullptr;   // (in the loop's body)
   long long n = 0;
   const bool prologue = part == kAll || part == kPrologue;
-  const int iterations = part == kAll ? opt.max_iterations : (part == kIteration ? 1 : 0);
+  const int iterations = part == kAll ? opt.max_iterations : (part == kIteration || part == kBody ? 1 : 0);
   size_t ev_i = 0;
   auto mark = [&](int stage) {
     if (!profile) return;
@@ -1954,8 +1987,10 @@ void Plan::enqueue(bool profile, Part part, cudaStream_t on, const cudaGraphCond
     // assembly do not read them, so they run beside them on a second
     // stream (the per-stage profile keeps one stream); a problem the control
     // stops only wastes that scratch work, as every later stage checks it.
-    const bool side = !profile && side_stream != nullptr;
-    if (side) {
+    const bool side = !profile && side_stream != nullptr && part != kBody;
+    if (part == kBody) {
+      // (done at the end of the last iteration, or by the prologue)
+    } else if (side) {
       GBA_CUDA(cudaEventRecord(ev_fork, s));
       GBA_CUDA(cudaStreamWaitEvent(side_stream, ev_fork, 0));
       n += launch_image_reduce(d, side_stream);
@@ -1977,7 +2012,7 @@ void Plan::enqueue(bool profile, Part part, cudaStream_t on, const cudaGraphCond
       mark(GBA_STAGE_OTHER);
       n += launch_pcg_setup(d, s);
       mark(GBA_STAGE_FACTOR);
-      n += launch_pcg_iterations(d, s, loop != nullptr);
+      n += launch_pcg_iterations(d, s, nested);
       mark(GBA_STAGE_SOLVE);
     } else {
       n += launch_assemble_S(d, s);
@@ -2000,11 +2035,11 @@ void Plan::enqueue(bool profile, Part part, cudaStream_t on, const cudaGraphCond
     n += launch_linearize(d, s, !d.fuse_lin);
     mark(GBA_STAGE_LINEARIZE);
   }
-  if (part == kAll || part == kEpilogue) {
-    if (part == kEpilogue || opt.max_iterations > 0) {
+  if (part == kAll || part == kEpilogue || part == kBody) {
+    if (part != kAll || opt.max_iterations > 0) {
       n += launch_image_reduce(d, s);
       mark(GBA_STAGE_IMAGE_REDUCE);
-      n += launch_ctrl_after_linearize(d, s);
+      n += launch_ctrl_after_linearize(d, s, loop);
       mark(GBA_STAGE_CONTROL);
     }
   }
@@ -2035,7 +2070,6 @@ int Plan::run() {
           enqueue(false, kPrologue);
           const long long pro = launches_last_run;
           capture_loop();
-          iter_launches = launches_last_run;
           launches_last_run += pro;
         } else {
           enqueue(profile);
