@@ -986,8 +986,9 @@ __device__ __forceinline__ void linearize_chunk(const DevPlan& d, const Chunk& c
       if (rws) {
         const float4 v = rws[k - ch.begin];
         rw[0] = v.x; rw[1] = v.y; rw[2] = v.z;
-      } else {
-        load_vec<4>(rwb + 4LL * k, rw);
+      } else {   // (k_cost_ff has just written them: not through the read-only path)
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(rwb + 4LL * k));
+        rw[0] = v.x; rw[1] = v.y; rw[2] = v.z;
       }
       if (d.x_ff[par]) {   // mixed: high part of the mirror
         const float2* xf = d.x_ff[par] + 3LL * pt;
