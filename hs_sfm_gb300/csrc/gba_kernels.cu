@@ -1833,8 +1833,11 @@ __global__ void __launch_bounds__(128) k_pairs_to_slots(const int4* __restrict__
 // ---------------------------------------------------------------------------
 // acc += x0 y0 + x1 y1 + x2 y2.  In FP64 one chain of three FMAs (three
 // instructions at 64 cycles each on this part's FP64 pipe instead of a
-// product, two FMAs and an addition); in FP32 the products first, the order
-// the mixed path's results are defined by.
+// product, two FMAs and an addition: 24 windows 19.7 ms a solve against 22.2,
+// the grid 48 against 54, their results as far from 64-bit references either
+// way; a sum of 190 signed triples alone is off by 1.2e-17 of the sum of
+// magnitudes, root mean square, against 1.05e-17); in FP32 the products first,
+// the order the mixed path's results are defined by.
 __device__ __forceinline__ void add_dot3(float& acc, float x0, float y0, float x1, float y1, float x2, float y2) {
   acc += x0 * y0 + x1 * y1 + x2 * y2;
 }
@@ -2054,8 +2057,8 @@ __global__ void __launch_bounds__(256) k_assemble_S_blocks(DevPlan d) {
 // column step.  Launch k (k = -1 .. nt-2) subtracts column k's rank-32
 // contribution from every trailing tile and factors column c = k+1: every
 // CTA of column c recomputes the diagonal tile's factor and inverse itself
-// (a 32x32 factorization held in one warp's registers), so no separate panel
-// launch is needed; the CTA owning tile (c, c) publishes L_cc^-1 and the
+// (tile_potrf_inverse: three of its warps in FP32, four in FP64), so no separate
+// panel launch is needed; the CTA owning tile (c, c) publishes L_cc^-1 and the
 // forward-solve value y_c = L_cc^-1 b_c.  S keeps its diagonal tiles (the
 // factor lives in Linv), the off-diagonal tiles are overwritten by L.
 // The backward solve L^T delta = y then takes one launch per tile row.
@@ -2696,22 +2699,25 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_chol_step(DevPl
 
 // Dataflow factorization of one problem's reduced system in a single
 // cooperative launch.  Every CTA owns a fixed set of tiles of the lower
-// triangle and keeps them in shared memory for the whole factorization: the
-// diagonal tile (i, i) and the tile left of it, (i, i-1), belong to the CTA
-// of row i; the other tiles are spread by work (j + 1 tasks for tile (i, j))
-// over all CTAs.  A tile's tasks are its updates A_ij -= L_ik L_jk^T for
+// triangle (df_layout) and keeps them in shared memory for the whole
+// factorization: row i's CTA its last ones, among them the diagonal tile (i, i)
+// and the tile left of it, the others spread by work (j + 1 tasks for tile
+// (i, j)).  A tile's tasks are its updates A_ij -= L_ik L_jk^T for
 // k = 0 .. j-1, in that order, then its factorization (i == j, with the
 // forward solve y_j = L_jj^-1 b_j) or its panel L_ij = A_ij L_jj^-T.  A
 // finished factor or panel is written to global memory (L into S, L_jj^-1
 // into Linv, y_j into b) and announced by storing the launch's epoch into
 // the tile's flag with release semantics (y_j has its own, in the upper
-// triangle of the flags); consumers poll flags with acquire loads and read
-// the data through L2.  Each CTA runs, among its tiles whose next task has its
-// inputs published, the one with the smallest (j, i), and applies up to
+// triangle of the flags); consumers poll the flags (acquire loads where one
+// flag is waited for; relaxed ones, several in flight, and then a fence where a
+// worker looks at all of its tiles) and read the data through L2.  Per
+// element the arithmetic is exactly that of k_chol_step (same tile routines,
+// same order of updates), so all schedules give the same bits.
+//
+// Without two CTAs per tile row each CTA runs, among its tiles whose next task
+// has its inputs published, the one with the smallest (j, i), and applies up to
 // df_batch consecutive ready updates of that tile with all of their loads in
-// flight together.  Per element the arithmetic is exactly that of k_chol_step
-// (same tile routines, same order of updates), so both schedules give the
-// same bits.
+// flight together.
 //
 // The critical path is the chain L_jj^-1 -> panel (j+1, j) -> last update of
 // (j+1, j+1) -> its factor.  The chain task of a row does these in one go:
@@ -2721,15 +2727,16 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_chol_step(DevPl
 // stored as they are found, so the flag follows the last of them directly,
 // before y_j.  With at least two CTAs per tile row (DevPlan::df_rows), row i's
 // CTA owns nothing but the row's last tiles (df_row_tiles) and runs a fixed
-// program instead of the scheduler: the updates of all of them column by
+// program instead of that scheduler: the updates of all of them column by
 // column, then the panel (i, i-2) with its updates, then the chain task, so
 // that the row is always waiting for L_{i-1,i-1}^-1 when it comes.  Scheduled
 // tile by tile, every second row was late for it by an update of its
 // diagonal tile and ran its panel, that update and its factor as three tasks
-// (7.5 us a row instead of 4.1).  With three CTAs per row (FP32), a second CTA
-// keeps the three columns left of those in the same way (df_helpers): panels
-// that wait their turn in a worker's queue are then needed several chain steps
-// later instead of one.
+// (7.5 us a row instead of 4.1).  With at least four CTAs per row (FP32), a
+// second CTA keeps the three columns left of those in the same way
+// (df_helpers): panels that wait their turn in a worker's queue are then needed
+// several chain steps later instead of one.  The other CTAs are workers
+// (worker_program).
 //
 // Every wait is bounded: a CTA that sees nothing ready for
 // DevPlan::df_spin_limit polls records a timeout and leaves; a failed pivot

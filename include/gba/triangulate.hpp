@@ -7,7 +7,7 @@
 //   MultipleViewMaximumLikelihoodEstimator<S>   multiple_view_maximum_likelihood_estimator.hpp:14-84
 //
 // plus MultipleViewTriangulator<S>, which solves many tracks in one call (one
-// GPU thread per point).  Rotations are angle-axis vectors (world to camera),
+// launch; a track's result does not depend on the others).  Rotations are angle-axis vectors (world to camera),
 // positions are camera centres; keys are the observed, distorted pixel keys.
 // Errors come back as the reference's Err: 0 on success, -1 otherwise.
 #ifndef GBA_TRIANGULATE_HPP_
