@@ -1657,8 +1657,11 @@ int Plan::build(const gba_problem* problems, const double* const* near_ys, int n
     if (v >= 0) D.solve_drop_step = v;
   }
   // Small FP32 systems: one factor-and-solve launch, a CTA per problem
-  // (GBA_CHOL_COLUMNS=1 keeps the per-column launches, for comparison).  A
-  // system alone on the device takes it up to four tile rows (21 images: 27 us
+  // (GBA_CHOL_COLUMNS=1 keeps the per-column launches, for comparison).  The
+  // launch's tiles are laid out for the plan's largest system, which decides
+  // for all: one of more than kSolveSmallTiles rows takes the whole batch to
+  // the per-column launches (the bound is the backward solve's, not the shared
+  // memory's; splitting a batch by size is not measured).  A system alone on the device takes it up to four tile rows (21 images: 27 us
   // against 34 for the dataflow launch and the solve; at five 35 against 39,
   // but its iteration is no faster, at eight 77 against 54).
   const bool dataflow = !pcg && nprob == 1 && !opt.shared_device && max_nt >= 2;

@@ -499,8 +499,8 @@ GBA_API int gba_cost_noalloc(const gba_device_problem* problem, int32_t loss,
  * (sfm_utility/camera_type.hpp): intrinsics [f skew cx cy pixel_ratio k1 k2
  * k3 d1 d2], extrinsics [rotation (angle-axis, world to camera), position
  * (the camera centre)].  Point j is seen by views track_views[t] with keys
- * track_keys[2t], t in [track_offsets[j], track_offsets[j+1]).  One thread
- * per point, FP64. */
+ * track_keys[2t], t in [track_offsets[j], track_offsets[j+1]).  FP64; a
+ * point's result does not depend on the other tracks. */
 typedef struct gba_triangulation {
   int64_t number_of_views;
   const double* intrinsics;       /* [10 V] */
