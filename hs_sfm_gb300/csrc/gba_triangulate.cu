@@ -28,7 +28,7 @@
 //    (about 200 instructions) instead of Jacobi sweeps (about 3,300), which
 //    remain for the systems where it does not settle.
 // 1M tracks of 2 to 12 views 24.3 -> 7.3 ms, 40,000 tracks 1.44 -> 0.47 ms,
-// 3,001 tracks of 2 to 8 views 0.41 -> 0.11 ms.
+// 3,001 tracks of 2 to 8 views 0.41 -> 0.095 ms.
 #include "gba_internal.h"
 
 #include <cmath>
