@@ -220,9 +220,9 @@ def load_tensor_peak():
 # DRAM bytes (read + write) per launch from one ncu capture of the grid
 # workload (profiles/k_*_grid_200cams_100kpts.md)
 NCU_DRAM_BYTES = {
-    ("grid", "factor"): 3.111168e6,
-    ("grid", "assemble"): 147.206912e6,
-    ("grid", "linearize"): 27.373568e6,
+    ("grid", "factor"): 3.162368e6,
+    ("grid", "assemble"): 129.868032e6,
+    ("grid", "linearize"): 28.396288e6,
 }
 
 
