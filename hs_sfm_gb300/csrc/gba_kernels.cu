@@ -1432,41 +1432,62 @@ __global__ void __launch_bounds__(256) k_image_reduce(DevPlan d) {
   }
 }
 
+// An image's items added up.  Mixed: a warp an image, the items in order.  FP64
+// (finer items, image_item_size): four interleaved compensated sums, a warp
+// each: five dependent additions an item at 64 cycles each, so with all four
+// in one warp and eight images to a CTA a window alone (40 items an image) took
+// 17 us longer a launch, 512 windows one after the other 283 solves/s instead of
+// 299.
+constexpr int kFinalizeThreads = 128;   // FP64: a CTA an image
+
+template <typename T>
 __global__ void __launch_bounds__(256) k_image_finalize(DevPlan d) {
-  const int img = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+  constexpr bool kWhole = sizeof(T) == sizeof(double);
+  constexpr long long kStride = kImageItemStride<T>;
+  __shared__ double sums[kWhole ? 4 : 1][2][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int img = kWhole ? int(blockIdx.x) : int(blockIdx.x) * 8 + warp;
   if (img >= d.I) return;
   const int prob = d.img_prob[img];
   const LMState& st = d.state[prob];
   if (!st.relin || !st.active) return;
   const int ib = d.img_item_off[img], ie = d.img_item_off[img + 1];
+  const double* part = d.img_item_partial + min(lane, 26);
   double v = 0.0;
-  if (lane < 27) {
-    const double* part = d.img_item_partial + lane;
-    if (d.precision == GBA_PRECISION_MIXED) {
-      for (int t = ib; t < ie; ++t) v += part[kImageItemStride<float> * t];
-    } else {   // finer items (image_item_size): four interleaved compensated sums
-      double s[4], c[4];
+  if constexpr (!kWhole) {
+    if (lane < 27)
+      for (int t = ib; t < ie; ++t) v += part[kStride * t];
+  } else {
+    double s = 0.0, c = 0.0;
+    for (int t0 = ib + warp; t0 < ie; t0 += 16) {
+      double hi[4], lo[4];   // (the loads of four items together)
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const double* p = part + kImageItemStride<double> * (ib + u);
-        s[u] = ib + u < ie ? p[0] : 0.0;
-        c[u] = ib + u < ie ? p[28] : 0.0;
+        const int t = min(t0 + 4 * u, ie - 1);
+        hi[u] = part[kStride * t];
+        lo[u] = part[kStride * t + 28];
       }
-      for (int t = ib + 4; t < ie; t += 4)
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (t + u < ie) {
-            const double* p = part + kImageItemStride<double> * (t + u);
-            const double y = p[0] + c[u], n = s[u] + y;
-            c[u] = (y - (n - s[u])) + p[28];
-            s[u] = n;
-          }
-      double e0, e1, e2;
-      const double a = two_sum(s[0], s[1], e0), b = two_sum(s[2], s[3], e1);
-      v = two_sum(a, b, e2);
-      v += ((c[0] + c[1]) + (c[2] + c[3])) + ((e0 + e1) + e2);
+      for (int u = 0; u < 4; ++u) {
+        if (u == 0 && t0 == ib + warp) {
+          s = hi[0];
+          c = lo[0];
+        } else if (t0 + 4 * u < ie) {
+          const double y = hi[u] + c, n = s + y;
+          c = (y - (n - s)) + lo[u];
+          s = n;
+        }
+      }
     }
+    sums[warp][0][lane] = s;
+    sums[warp][1][lane] = c;
+    __syncthreads();
+    if (warp > 0) return;
+    double e0, e1, e2;
+    const double a = two_sum(sums[0][0][lane], sums[1][0][lane], e0),
+                 b = two_sum(sums[2][0][lane], sums[3][0][lane], e1);
+    v = two_sum(a, b, e2);
+    v += ((sums[0][1][lane] + sums[1][1][lane]) + (sums[2][1][lane] + sums[3][1][lane])) + ((e0 + e1) + e2);
   }
   // lane e holds entry e of (upper U in row order, then g)
   double* U = d.U + 36LL * img;
@@ -4867,7 +4888,10 @@ int launch_linearize(const DevPlan& d, cudaStream_t s, bool keys) {
 int launch_image_reduce(const DevPlan& d, cudaStream_t s) {
   if (d.n_img_items <= 0) return 0;
   GBA_DISPATCH(d, (k_image_reduce<T><<<(d.n_img_items + 7) / 8, 256, 0, s>>>(d)));
-  k_image_finalize<<<(d.I + 7) / 8, 256, 0, s>>>(d);
+  if (d.precision == GBA_PRECISION_MIXED)
+    k_image_finalize<float><<<(d.I + 7) / 8, 256, 0, s>>>(d);
+  else
+    k_image_finalize<double><<<d.I, kFinalizeThreads, 0, s>>>(d);
   if (!d.free_cams) return 2;
   GBA_DISPATCH(d, (k_image_cam_reduce<T><<<d.n_img_items, 128, 0, s>>>(d)));
   k_image_cam_finalize<<<d.I, kImgCamVals, 0, s>>>(d);
